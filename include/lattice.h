@@ -101,8 +101,10 @@ typedef struct lat_config {
 /* How a spectral kick computes its Laplacian.  CUFFT: 3D R2C, -k^2/N multiply
  * and C2R (any size).  SEPARABLE: three passes of in-register 1D transforms,
  * one per axis (sides 16..512, powers of two), which also transform the FP32
- * field with its Kahan compensation.  AUTO: cuFFT until lat_autotune times
- * both on the handle's lattice and keeps the faster. */
+ * field with its Kahan compensation.  AUTO: until lat_autotune times both on
+ * the handle's lattice and keeps the faster, FP64 lattices with power-of-two
+ * sides 16..512 run the passes (two fields: any such sides; one field: nx >=
+ * 64), all others cuFFT. */
 enum lat_spectral_impl { LAT_SPEC_IMPL_AUTO = 0, LAT_SPEC_IMPL_CUFFT = 1, LAT_SPEC_IMPL_SEPARABLE = 2 };
 
 typedef struct lat_s lat_t;

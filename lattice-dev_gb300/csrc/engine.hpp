@@ -126,6 +126,7 @@ struct SepArgs {
   float* shift_a;           // [2 * pairs] shift of zs per run: written by pass X, read by pass Z
   float* shift_b;           // [2 * pairs] phi at site 0 of each run: written by pass Z, read by pass X
   int* grid_out;            // host: receives the grid of a streamed pass (or null)
+  int nan_flag;             // fixed-point passes: a non-finite field sets the NaN flag
   DevScalars* sc;
   RedBuf rb;
   // streamed passes Y and Z: tensor maps of zs (float, dims {2 nx, ny, nz,
@@ -138,12 +139,19 @@ struct SepArgs {
 // Encode the two tensor maps of a streamed pass along `axis` (1 or 2) with
 // `lines` x-columns per tile and line length n.
 int encode_stream_tmaps(SepArgs& a, int axis, int lines, int n);
-int launch_sep_16(const SepArgs& a, int precision, int axis, cudaStream_t s);
-int launch_sep_32(const SepArgs& a, int precision, int axis, cudaStream_t s);
-int launch_sep_64(const SepArgs& a, int precision, int axis, cudaStream_t s);
-int launch_sep_128(const SepArgs& a, int precision, int axis, cudaStream_t s);
-int launch_sep_256(const SepArgs& a, int precision, int axis, cudaStream_t s);
-int launch_sep_512(const SepArgs& a, int precision, int axis, cudaStream_t s);
+int launch_sep_16(const SepArgs& a, int axis, cudaStream_t s);
+int launch_sep_32(const SepArgs& a, int axis, cudaStream_t s);
+int launch_sep_64(const SepArgs& a, int axis, cudaStream_t s);
+int launch_sep_128(const SepArgs& a, int axis, cudaStream_t s);
+int launch_sep_256(const SepArgs& a, int axis, cudaStream_t s);
+int launch_sep_512(const SepArgs& a, int axis, cudaStream_t s);
+// FP64 passes with fixed-point line transforms (k_fx.cuh), in place
+int launch_fx_16(const SepArgs& a, int axis, cudaStream_t s);
+int launch_fx_32(const SepArgs& a, int axis, cudaStream_t s);
+int launch_fx_64(const SepArgs& a, int axis, cudaStream_t s);
+int launch_fx_128(const SepArgs& a, int axis, cudaStream_t s);
+int launch_fx_256(const SepArgs& a, int axis, cudaStream_t s);
+int launch_fx_512(const SepArgs& a, int axis, cudaStream_t s);
 int sep_stream_lines_128(int axis);  // lines per tile of the streamed passes (k_sep_stream.cuh)
 int sep_stream_lines_256(int axis);
 // streamed passes over pairs of one-field runs (ensembles), lines of n = 64,

@@ -1,4 +1,5 @@
-// k_sep.cuh -- separable spectral Laplacian passes (sm_103a).
+// k_sep.cuh -- separable spectral Laplacian passes of FP32-Kahan lattices
+// (sm_103a); FP64 lattices run the fixed-point passes of k_fx.cuh.
 //
 // The spectral Laplacian of laplacian_3d (Pseudospec/openmp_dev/fftw_mod.f90:
 // 177-207: r2c, multiply by -(ii^2+jj^2+kk^2) dk^2, c2r, divide by N) is a
@@ -53,12 +54,6 @@ template <> struct Cx<float> {
   static __device__ __forceinline__ float2 tw(int j) { return make_float2(c_tw64f[j][0], c_tw64f[j][1]); }
   static __device__ __forceinline__ float2 tw24(int j) { return make_float2(c_tw24f[j][0], c_tw24f[j][1]); }
 };
-template <> struct Cx<double> {
-  using T = double2;
-  static __device__ __forceinline__ double2 tw(int j) { return make_double2(c_tw64[j][0], c_tw64[j][1]); }
-  static __device__ __forceinline__ double2 tw24(int j) { return make_double2(c_tw24[j][0], c_tw24[j][1]); }
-};
-
 template <typename C> __device__ __forceinline__ C cmul(C a, C b) {
   C r;
   r.x = a.x * b.x - a.y * b.y;
@@ -676,20 +671,15 @@ int sep_go(const SepArgs& a, cudaStream_t s) {
 }
 
 template <int N>
-int sep_dispatch(const SepArgs& a, int precision, int axis, cudaStream_t s) {
+int sep_dispatch(const SepArgs& a, int axis, cudaStream_t s) {
 #define LAT_SEP_AX(R, NF, K)                                    \
   switch (axis) {                                                \
     case 0: return sep_go<R, NF, 0, N, K>(a, s);                \
     case 1: return sep_go<R, NF, 1, N, K>(a, s);                \
     default: return sep_go<R, NF, 2, N, K>(a, s);               \
   }
-  if (precision == LAT_FP64) {
-    if (a.nf == 1) { LAT_SEP_AX(double, 1, false) }
-    else { LAT_SEP_AX(double, 2, false) }
-  } else {
-    if (a.nf == 1) { LAT_SEP_AX(float, 1, true) }
-    else { LAT_SEP_AX(float, 2, true) }
-  }
+  if (a.nf == 1) { LAT_SEP_AX(float, 1, true) }
+  LAT_SEP_AX(float, 2, true)
 #undef LAT_SEP_AX
 }
 

@@ -2,8 +2,8 @@
 #include "k_sep_stream.cuh"
 
 namespace lat {
-int launch_sep_64(const SepArgs& a, int precision, int axis, cudaStream_t s) {
-  return sep::sep_dispatch<64>(a, precision, axis, s);
+int launch_sep_64(const SepArgs& a, int axis, cudaStream_t s) {
+  return sep::sep_dispatch<64>(a, axis, s);
 }
 int sep_columns_64(int precision, int nf) { return sep::sep_columns<64>(precision, nf); }
 // pairs of one-field runs (ensembles)
