@@ -131,7 +131,9 @@ struct lat_s {
   bool sep = false;               // and in use
   bool fx_ok = false;             // FP64: the fixed-point passes (k_fx.cuh) tile these sizes
   bool sep_stream = true;         // streamed passes where available (LAT_SEP_CLASSIC=1: off)
-  void* tw[3] = {nullptr, nullptr, nullptr};  // W_N^j per axis, field precision
+  void* tw[3] = {nullptr, nullptr, nullptr};  // W_N^j per axis, FP32 (k_sep.cuh)
+  fx::Tw* fxtw[3] = {nullptr, nullptr, nullptr};  // and as split integers (one allocation): sides the fixed-point
+                                                  // transforms take, else null
 
   int fd_ty = 8, fd_zc = 32;
   int pw_grid = 0, pw_block = 256;
@@ -236,6 +238,9 @@ int n_terms(const lat_s* h) {
   return conformal(h) ? 3 : 2;
 }
 
+// line lengths of the separable passes and of the fixed-point transforms
+bool fx_side(int n) { return n >= 16 && n <= 512 && (n & (n - 1)) == 0; }
+
 // Whether an AUTO lattice takes the separable passes before any autotuning:
 // FP64 lattices that the fixed-point passes tile.  A Yoshida-4 step of two
 // expanding fields: 0.12 ms against 0.24 ms on cuFFT at 32^3, 4.8 against 24.8
@@ -262,6 +267,36 @@ int fft_exec_c2r(lat_s* h, cufftHandle p, void* in, void* out) {
   Timed t(h, LAT_K_FFT_C2R);
   if (h->prec == LAT_FP64) CF(cufftExecZ2D(p, (cufftDoubleComplex*)in, (cufftDoubleReal*)out));
   else CF(cufftExecC2R(p, (cufftComplex*)in, (cufftReal*)out));
+  return LAT_OK;
+}
+
+// Forward transform of one FP64 array, or of one FP32 array with its
+// compensation (phi_hi - c), into the half spectrum F [nz][ny][nx/2+1] of
+// complex FP64, in fixed point; the lattice must have its tables (fxtw).
+int fx_r2c(lat_s* h, const void* hi, const void* c, double2* F) {
+  Timed t(h, LAT_K_FFT_R2C);
+  const int hx = h->nx / 2 + 1;
+  const int64_t plane = (int64_t)hx * h->ny;
+#define LAT_FXR(n, call)                            \
+  switch (n) {                                      \
+    case 16: RET(launch_fxr_##call(16)); break;     \
+    case 32: RET(launch_fxr_##call(32)); break;     \
+    case 64: RET(launch_fxr_##call(64)); break;     \
+    case 128: RET(launch_fxr_##call(128)); break;   \
+    case 256: RET(launch_fxr_##call(256)); break;   \
+    case 512: RET(launch_fxr_##call(512)); break;   \
+    default: return set_error(LAT_ERR_STATE, "fixed-point transform: line length"); \
+  }
+#define launch_fxr_rows(N_) launch_fxr_rows_##N_(hi, c, h->prec, F, (int64_t)h->ny * h->nz / 2, h->fxtw[0], h->nsm, h->stream)
+#define launch_fxr_y(N_) launch_fxr_lines_##N_(F, (int64_t)hx * h->nz, hx, plane, hx, h->fxtw[1], h->nsm, h->stream)
+#define launch_fxr_z(N_) launch_fxr_lines_##N_(F, plane, (int)plane, 0, plane, h->fxtw[2], h->nsm, h->stream)
+  LAT_FXR(h->nx, rows)
+  LAT_FXR(h->ny, y)
+  LAT_FXR(h->nz, z)
+#undef launch_fxr_rows
+#undef launch_fxr_y
+#undef launch_fxr_z
+#undef LAT_FXR
   return LAT_OK;
 }
 
@@ -603,7 +638,7 @@ int sep_pass(lat_s* h, int axis, double hk, double hg, double hd, int* grid_out 
     a.lap = axis == 2 ? h->lap_alt : h->lap;
     a.lap_out = axis == 0 ? h->lap : h->lap_alt;
   }
-  a.twN = h->tw[axis];
+  a.twN = fx ? static_cast<const void*>(h->fxtw[axis]) : h->tw[axis];
   if (!(fx ? h->fx_ok : h->sep_ok) || !a.twN || !a.phi || !a.phi_out || !a.pi || !a.pi_out || !a.lap || !a.lap_out ||
       (h->prec == LAT_FP32_KAHAN && (!a.phic || !a.phic_out)))
     return set_error(LAT_ERR_STATE, "separable pass buffers missing");
@@ -954,7 +989,12 @@ int compute_energies(lat_s* h, double* out, double ball_r2 = 0.0, double* ball =
     RET(launch_energy(e, h->prec, h->stream));
   }
   if (spectral(h)) {
-    RET(fft_exec_r2c(h, h->p_r2c, h->fld[h->cur], h->Fk));
+    if (h->prec == LAT_FP64 && h->fxtw[0]) {
+      for (int l = 0; l < h->nf; ++l)
+        RET(fx_r2c(h, (const double*)h->fld[h->cur] + l * h->N, nullptr, (double2*)h->Fk + l * h->M));
+    } else {
+      RET(fft_exec_r2c(h, h->p_r2c, h->fld[h->cur], h->Fk));
+    }
     Timed t(h, LAT_K_OTHER);
     RET(launch_parseval(h->Fk, h->nx, h->ny, h->nz, h->nf, h->dkx * h->dkx, h->dky * h->dky, h->dkz * h->dkz,
                         h->sc, 8, red(h), h->pw_grid, h->prec, h->stream));
@@ -1038,12 +1078,21 @@ int output_spectrum(lat_s* h, int what, int field, int slot, void** Fout, int* p
   RET(src_ptr(h, what, field, &src));
   if (h->prec == LAT_FP64) {
     void* F = (char*)h->Fk + (size_t)slot * h->M * h->csz;
-    RET(fft_exec_r2c(h, h->p_r2c1, src, F));
+    if (h->fxtw[0]) RET(fx_r2c(h, src, nullptr, static_cast<double2*>(F)));
+    else RET(fft_exec_r2c(h, h->p_r2c1, src, F));
     *Fout = F;
     *prec = LAT_FP64;
     return LAT_OK;
   }
   if (!h->Fk64) CK(cudaMalloc(&h->Fk64, (size_t)2 * h->M * sizeof(double2)));
+  if (h->fxtw[0]) {
+    const void* cmp = (what == LAT_SPEC_FLD && h->fldc) ? (const char*)h->fldc + (size_t)field * h->N * h->rsz : nullptr;
+    double2* F = static_cast<double2*>(h->Fk64) + (size_t)slot * h->M;
+    RET(fx_r2c(h, src, cmp, F));
+    *Fout = F;
+    *prec = LAT_FP64;
+    return LAT_OK;
+  }
   if (!h->have_d2z1) {
     CF(cufftCreate(&h->p_d2z1));
     int n[3] = {h->nz, h->ny, h->nx};
@@ -1182,6 +1231,7 @@ int lat_destroy(lat_t* h) {
   if (h->cl_stream) cudaStreamDestroy(h->cl_stream);
   for (void* t : h->tw)
     if (t) cudaFree(t);
+  if (h->fxtw[0]) cudaFree(h->fxtw[0]);
   {
     void* cb[] = {h->cl_b.a0, h->cl_b.a1, h->cl_b.a2, h->cl_b.out};
     for (void* b : cb)
@@ -1307,7 +1357,6 @@ int lat_create(lat_t** out, const lat_config* cfg) {
     if ((st = make_plan(h, &h->p_c2r, &h->have_c2r, false, h->nf))) return bail(st);
   }
   if (spectral(h)) {
-    auto pow2ok = [](int n) { return n >= 16 && n <= 512 && (n & (n - 1)) == 0; };
     auto cols = [&](int n) {  // x-columns per block of a y or z pass of length n
       switch (n) {
         case 16: return sep_columns_16(h->prec, h->nf);
@@ -1318,13 +1367,13 @@ int lat_create(lat_t** out, const lat_config* cfg) {
         default: return sep_columns_512(h->prec, h->nf);
       }
     };
-    h->sep_ok = pow2ok(h->nx) && pow2ok(h->ny) && pow2ok(h->nz);
+    h->sep_ok = fx_side(h->nx) && fx_side(h->ny) && fx_side(h->nz);
     // the passes need whole column blocks and (one field) an even number of x-rows
     if (h->sep_ok) h->sep_ok = h->nx % cols(h->ny) == 0 && h->nx % cols(h->nz) == 0;
     if (cfg->spectral_impl == LAT_SPEC_IMPL_SEPARABLE && !h->sep_ok)
       return bail(set_error(LAT_ERR_UNSUPPORTED, "separable spectral passes need power-of-two sides 16..512"));
     // FP64: 16 complex lines per tile (x-columns: 16 with two fields, 32 with one)
-    h->fx_ok = h->prec == LAT_FP64 && pow2ok(h->nx) && pow2ok(h->ny) && pow2ok(h->nz) &&
+    h->fx_ok = h->prec == LAT_FP64 && fx_side(h->nx) && fx_side(h->ny) && fx_side(h->nz) &&
                h->nx % (h->nf == 2 ? 16 : 32) == 0;
     h->sep = h->sep_ok && cfg->spectral_impl == LAT_SPEC_IMPL_SEPARABLE && !getenv_flag("LAT_NO_SEPARABLE");
     if (cfg->spectral_impl == LAT_SPEC_IMPL_AUTO) h->sep = auto_separable(h);
@@ -1343,32 +1392,43 @@ int lat_create(lat_t** out, const lat_config* cfg) {
       if ((st = alloc(&h->fldp_alt, fb))) return bail(st);
       if ((st = alloc(&h->lap_alt, fb))) return bail(st);
     }
-    if (h->sep_ok || h->fx_ok) {  // the autotuner may switch an AUTO handle to the passes later
+    if (h->sep_ok && h->prec != LAT_FP64) {  // the autotuner may switch an AUTO handle to the passes later
       const int dims[3] = {h->nx, h->ny, h->nz};
       for (int ax = 0; ax < 3; ++ax) {
         const int n = dims[ax];
         std::vector<float> w32(2 * n);
-        std::vector<int> wfx(4 * n);
         for (int j = 0; j < n; ++j) {
           const long double ang = -6.283185307179586476925286766559L * (long double)j / (long double)n;
-          const long double c = cosl(ang), sn = sinl(ang);
-          w32[2 * j] = (float)(double)c;
-          w32[2 * j + 1] = (float)(double)sn;
-          const long double one = 4611686018427387904.0L;  // 2^62
-          const long long ci = llrintl(c * one), si = llrintl(sn * one);
-          wfx[4 * j] = fx::split_hi(ci);
-          wfx[4 * j + 1] = fx::split_lo(ci);
-          wfx[4 * j + 2] = fx::split_hi(si);
-          wfx[4 * j + 3] = fx::split_lo(si);
+          w32[2 * j] = (float)(double)cosl(ang);
+          w32[2 * j + 1] = (float)(double)sinl(ang);
         }
-        const size_t bytes = h->prec == LAT_FP64 ? wfx.size() * sizeof(int) : w32.size() * sizeof(float);
-        if ((st = alloc(&h->tw[ax], bytes))) return bail(st);
-        const void* src = h->prec == LAT_FP64 ? (const void*)wfx.data() : (const void*)w32.data();
-        if ((e = cudaMemcpyAsync(h->tw[ax], src, bytes, cudaMemcpyHostToDevice, h->stream)) != cudaSuccess)
+        if ((st = alloc(&h->tw[ax], w32.size() * sizeof(float)))) return bail(st);
+        if ((e = cudaMemcpyAsync(h->tw[ax], w32.data(), w32.size() * sizeof(float), cudaMemcpyHostToDevice,
+                                 h->stream)) != cudaSuccess)
           return bail(cuda_fail(e, "twiddle upload"));
         if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return bail(cuda_fail(e, "twiddle upload"));
       }
     }
+  }
+  if (fx_side(h->nx) && fx_side(h->ny) && fx_side(h->nz)) {
+    const int dims[3] = {h->nx, h->ny, h->nz};
+    std::vector<fx::Tw> w((size_t)h->nx + h->ny + h->nz);
+    if ((st = alloc((void**)&h->fxtw[0], w.size() * sizeof(fx::Tw)))) return bail(st);
+    size_t at = 0;
+    for (int ax = 0; ax < 3; ++ax) {
+      h->fxtw[ax] = h->fxtw[0] + at;
+      for (int j = 0; j < dims[ax]; ++j) {
+        const long double ang = -6.283185307179586476925286766559L * (long double)j / (long double)dims[ax];
+        const long double one = 4611686018427387904.0L;  // 2^62
+        const long long c = llrintl(cosl(ang) * one), sn = llrintl(sinl(ang) * one);
+        w[at + j] = fx::Tw{fx::split_hi(c), fx::split_lo(c), fx::split_hi(sn), fx::split_lo(sn)};
+      }
+      at += dims[ax];
+    }
+    if ((e = cudaMemcpyAsync(h->fxtw[0], w.data(), w.size() * sizeof(fx::Tw), cudaMemcpyHostToDevice, h->stream)) !=
+            cudaSuccess ||
+        (e = cudaStreamSynchronize(h->stream)) != cudaSuccess)
+      return bail(cuda_fail(e, "twiddle upload"));
   }
   h->ev_pool.resize(4096);
   for (auto& ev : h->ev_pool) {
@@ -1652,8 +1712,13 @@ int lat_gw_spectrum(lat_t* h, int32_t nbins, double* S, double* W) {
   if (nbins < 1 || nbins > kMaxBins) return set_error(LAT_ERR_ARG, "nbins out of range");
   ApiGuard g(h);
   if (!h->Fk6) CK(cudaMalloc(&h->Fk6, (size_t)6 * h->M * h->csz));
-  RET(make_plan(h, &h->p_r2c6, &h->have_r2c6, true, 6));
-  RET(fft_exec_r2c(h, h->p_r2c6, h->pu, h->Fk6));
+  if (h->prec == LAT_FP64 && h->fxtw[0]) {
+    for (int k = 0; k < 6; ++k)
+      RET(fx_r2c(h, (const double*)h->pu + k * h->N, nullptr, (double2*)h->Fk6 + k * h->M));
+  } else {
+    RET(make_plan(h, &h->p_r2c6, &h->have_r2c6, true, 6));
+    RET(fft_exec_r2c(h, h->p_r2c6, h->pu, h->Fk6));
+  }
   GwSpecArgs a{};
   a.nx = h->nx; a.ny = h->ny; a.nz = h->nz;
   for (int c = 0; c < 6; ++c) a.F[c] = (const char*)h->Fk6 + (size_t)c * h->M * h->csz;

@@ -152,6 +152,31 @@ int launch_fx_64(const SepArgs& a, int axis, cudaStream_t s);
 int launch_fx_128(const SepArgs& a, int axis, cudaStream_t s);
 int launch_fx_256(const SepArgs& a, int axis, cudaStream_t s);
 int launch_fx_512(const SepArgs& a, int axis, cudaStream_t s);
+// 3D real-to-complex transform in fixed point (k_fxr.cuh): rows, then lines along y and z
+int launch_fxr_rows_16(const void* hi, const void* c, int precision, void* F, int64_t nlines, const void* tw, int nsm,
+                       cudaStream_t s);
+int launch_fxr_lines_16(void* F, int64_t nlines, int per, int64_t plane, int64_t stride, const void* tw, int nsm,
+                        cudaStream_t s);
+int launch_fxr_rows_32(const void* hi, const void* c, int precision, void* F, int64_t nlines, const void* tw, int nsm,
+                       cudaStream_t s);
+int launch_fxr_lines_32(void* F, int64_t nlines, int per, int64_t plane, int64_t stride, const void* tw, int nsm,
+                        cudaStream_t s);
+int launch_fxr_rows_64(const void* hi, const void* c, int precision, void* F, int64_t nlines, const void* tw, int nsm,
+                       cudaStream_t s);
+int launch_fxr_lines_64(void* F, int64_t nlines, int per, int64_t plane, int64_t stride, const void* tw, int nsm,
+                        cudaStream_t s);
+int launch_fxr_rows_128(const void* hi, const void* c, int precision, void* F, int64_t nlines, const void* tw, int nsm,
+                       cudaStream_t s);
+int launch_fxr_lines_128(void* F, int64_t nlines, int per, int64_t plane, int64_t stride, const void* tw, int nsm,
+                        cudaStream_t s);
+int launch_fxr_rows_256(const void* hi, const void* c, int precision, void* F, int64_t nlines, const void* tw, int nsm,
+                       cudaStream_t s);
+int launch_fxr_lines_256(void* F, int64_t nlines, int per, int64_t plane, int64_t stride, const void* tw, int nsm,
+                        cudaStream_t s);
+int launch_fxr_rows_512(const void* hi, const void* c, int precision, void* F, int64_t nlines, const void* tw, int nsm,
+                       cudaStream_t s);
+int launch_fxr_lines_512(void* F, int64_t nlines, int per, int64_t plane, int64_t stride, const void* tw, int nsm,
+                        cudaStream_t s);
 int sep_stream_lines_128(int axis);  // lines per tile of the streamed passes (k_sep_stream.cuh)
 int sep_stream_lines_256(int axis);
 // streamed passes over pairs of one-field runs (ensembles), lines of n = 64,

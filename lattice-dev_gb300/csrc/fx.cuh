@@ -231,6 +231,7 @@ LAT_HD void dft(i64 (&re)[R], i64 (&im)[R]) {
 
 // ------------------------------------------------------------ conversions
 constexpr int kNanExp = 2047;
+constexpr u64 kNan = 0x7ff8000000000000ULL;
 
 LAT_HD int exp_of(u64 b) {  // biased exponent, subnormals with the smallest
   const int e = (int)(b >> 52) & 0x7ff;
@@ -277,6 +278,19 @@ LAT_HD u64 to_bits(i64 v) {
   const unsigned int e = top ? (unsigned int)(1023 - sh) << 20 : 0u;  // the leading bit adds one
   return (m + ((u64)e << 32)) | ((u64)s & 0x8000000000000000ULL);
 }
+// v 2^(e - 61) rounded to FP64, |v| < 2^63; below the normal range 0, above it infinite
+LAT_HD u64 to_bits_exp(i64 v, int e) {
+  const i64 s = v >> 63;
+  u64 m = (u64)((v ^ s) - s);
+  const unsigned int hi = (unsigned int)(m >> 32), top = hi ? hi : (unsigned int)m;
+  const int sh = lead0(top) + (hi ? -1 : 31);
+  m = ((m << sh) + 0x200) >> 10;
+  const int ex = 1023 - sh + e;  // the leading bit adds one
+  u64 r = m + ((u64)(unsigned int)ex << 52);
+  r = ex > 2045 ? 0x7ff0000000000000ULL : r;
+  r = (top == 0 || ex < 0) ? 0 : r;
+  return r | ((u64)s & 0x8000000000000000ULL);
+}
 LAT_HD double bits_double(u64 b) {
 #ifdef __CUDA_ARCH__
   return __longlong_as_double((i64)b);
@@ -316,13 +330,16 @@ template <> struct Split<512> { static constexpr int P = 16, Q = 32, LOG = 9; };
 struct LineBits {
   int nm, ns;
 };
-template <int N>
+template <int N, int LOG = Split<N>::LOG>
 LAT_HD LineBits line_bits(u64 ored, u64 sum) {
-  const int nm = 64 - clz64(ored), ns = 64 - clz64(sum) + 9, top = nm + Split<N>::LOG;
+  const int nm = 64 - clz64(ored), ns = 64 - clz64(sum) + 9, top = nm + LOG;
   return LineBits{nm, ns < top ? ns : top};
 }
 // deviations scaled so that their sum stays below 2^61
 LAT_HD i64 scale_line(i64 d, LineBits b) { return shl(d, 63 - b.nm) >> (2 + b.ns - b.nm); }
+// exponent of a scaled line's unit times 2^61 (to_bits_exp); emax the largest
+// biased exponent of the line
+LAT_HD int emax_unit(int emax, LineBits b) { return emax - 1084 + b.ns; }
 // Bits to drop at the multiplier so that N times the largest value of either
 // line stays below 2^61.  A line whose sum is close to its largest value (a
 // spike) needs up to log2 N; dropping more than four would cost the other
@@ -342,9 +359,9 @@ LAT_HD int drop_bits(LineBits& a, LineBits& b) {
 // ns + drop), emax the largest biased exponent of the line.  Exactly zero for a constant line, NaN
 // for one that holds a NaN or an infinity.
 LAT_HD double line_coef(double c, int emax, LineBits b, int drop) {
-  if (emax == kNanExp) return bits_double(0x7ff8000000000000ULL);
+  if (emax == kNanExp) return bits_double(kNan);
   if (b.nm == 0) return 0.0;
-  return pow2_times(c, emax - 1084 + b.ns + drop);
+  return pow2_times(c, emax_unit(emax, b) + drop);
 }
 
 // The line transform in three phases; a barrier over the line's threads
@@ -392,6 +409,27 @@ LAT_HD void phase2(int t, Cx64* sl, const Tw* t2, int drop) {
       sl[kq * S + m] = Cx64{ur[m], ui[m]};
     });
   });
+}
+// Forward transform only: row kq of the scratch becomes Z[kq + Q kp], kp < P
+// (after phase 1 and a barrier; each row belongs to one thread).
+template <int N>
+LAT_HD void phase2_forward(int t, Cx64* sl) {
+  constexpr int P = Split<N>::P, Q = Split<N>::Q, S = P + 1, G = Q / P;
+  static_for<G>([&](auto gg) {
+    const int kq = t + gg.value * P;
+    i64 ur[P], ui[P];
+    static_for<P>([&](auto tt) {
+      const Cx64 z = sl[kq * S + tt.value];
+      ur[tt.value] = z.x;
+      ui[tt.value] = z.y;
+    });
+    dft<P, false>(ur, ui);
+    static_for<P>([&](auto kp) { sl[kq * S + kp.value] = Cx64{ur[kp.value], ui[kp.value]}; });
+  });
+}
+template <int N>
+LAT_HD const Cx64& mode_at(const Cx64* sl, int k) {
+  return sl[(k % Split<N>::Q) * (Split<N>::P + 1) + k / Split<N>::Q];
 }
 template <int N>
 LAT_HD void phase3(i64 (&re)[Split<N>::Q], i64 (&im)[Split<N>::Q], int t, const Cx64* sl) {

@@ -108,3 +108,30 @@ def test_evolution_is_reproducible(engine):
         a.symp(4, 0.01, 4)
         out.append((*a.get_state(), a.scale_factor()))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1]) and out[0][2] == out[1][2]
+
+
+@pytest.mark.parametrize("prec", [L.FP64, L.FP32_KAHAN])
+@pytest.mark.parametrize("shape", [(16, 16, 16), (16, 512, 32), (512, 32, 16), (32, 16, 512), (64, 128, 256)])
+def test_spectrum_transform_matches_numpy(engine, shape, prec):
+    """The fixed-point real-to-complex transform under the spectra (csrc/k_fxr.cuh), every line
+    length along every axis, against numpy's FP64 transform of the same numbers binned like
+    spectrum_bin; each bin is a sum of squares, so FP64 rounding leaves it within 1e-11."""
+    nx, ny, nz = shape
+    c = L.make_config(shape, nfld=1, length=1.0 * nx, laplacian=L.LAP_FD7, precision=prec)
+    g = engine.Lattice(c)
+    f, p = random_state((1, nz, ny, nx), seed=21, mean=3.0, amp=1e-3)
+    g.set_state(f, p)
+    x, y = g.get_state()  # what the handle holds (FP32-Kahan: phi_hi - c)
+    nb = g.nbins()
+    fold = [np.minimum(np.arange(n), n - np.arange(n)) for n in (nz, ny)] + [np.arange(nx // 2 + 1)]
+    m2 = fold[0][:, None, None] ** 2 + fold[1][None, :, None] ** 2 + fold[2][None, None, :] ** 2
+    l = np.floor(np.sqrt(m2)).astype(int).ravel()
+    w = np.broadcast_to(np.where((fold[2] == 0) | (2 * fold[2] == nx), 1.0, 2.0), m2.shape).ravel()
+    for what, a in ((L.SPEC_FLD, x[0]), (L.SPEC_FLDP, y[0])):
+        F = np.fft.rfftn(a)
+        S = np.bincount(l, w * (F.real ** 2 + F.imag ** 2).ravel(), nb)[:nb]
+        W = np.bincount(l, w, nb)[:nb]
+        got, cnt = g.spectrum_bin(what, 0, nb)
+        assert np.array_equal(cnt, W)
+        ok = W > 0
+        assert np.max(np.abs(got[ok] * W[ok] / S[ok] - 1)) <= 1e-11
