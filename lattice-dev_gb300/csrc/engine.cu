@@ -22,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "bin.hpp"
 #include "engine.hpp"
 #include "fx.cuh"
 #include "integrator.hpp"
@@ -109,10 +110,7 @@ struct lat_s {
   DevScalars* sc = nullptr;
   RedBuf rb{};
   int64_t red_cap = 0;  // blocks the partial buffer holds
-  double* spec_part = nullptr;
-  double* spec_out = nullptr;
-  unsigned int* spec_counter = nullptr;
-  int spec_grid = 0;
+  BinPlan bins;         // spectra of this lattice shape
   double* stage = nullptr;  // nf*N doubles
   size_t stage_elems = 0;
 
@@ -1049,26 +1047,6 @@ int src_ptr(lat_s* h, int what, int field, const void** p) {
   return LAT_OK;
 }
 
-int run_spectrum(lat_s* h, const void* F1, const void* F2, int mode, int nbins, double* hostout, int prec) {
-  SpecArgs s{};
-  s.nx = h->nx; s.ny = h->ny; s.nz = h->nz;
-  s.F1 = F1; s.F2 = F2; s.mode = mode; s.nbins = nbins;
-  s.partials = h->spec_part;
-  s.out = h->spec_out;
-  s.counter = h->spec_counter;
-  s.grid = h->spec_grid;
-  s.block = 256;
-  {
-    Timed t(h, LAT_K_OTHER);
-    RET(launch_spectrum(s, prec, h->stream));
-  }
-  CK(cudaMemcpyAsync(hostout, h->spec_out, sizeof(double) * 3 * nbins, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
-  return LAT_OK;
-}
-
-const int kMaxBins = 2048;
-
 // Half spectrum of one field or momentum array for the output routines.  An
 // FP32 field is transformed in FP64 from phi_hi - c, so a field sitting near
 // a large mean keeps the digits of its fluctuation (an FP32 transform of
@@ -1232,6 +1210,7 @@ int lat_destroy(lat_t* h) {
   for (void* t : h->tw)
     if (t) cudaFree(t);
   if (h->fxtw[0]) cudaFree(h->fxtw[0]);
+  h->bins.free();
   {
     void* cb[] = {h->cl_b.a0, h->cl_b.a1, h->cl_b.a2, h->cl_b.out};
     for (void* b : cb)
@@ -1241,7 +1220,7 @@ int lat_destroy(lat_t* h) {
   if (h->have_d2z1) cufftDestroy(h->p_d2z1);
   void* bufs[] = {h->fld[0], h->fld[1], h->fldc, h->fldp, h->lap, h->fldc_alt, h->fldp_alt, h->lap_alt, h->Fk,
                   h->u[0], h->u[1], h->pu, h->Fk6,
-                  h->sc, h->rb.partials, h->rb.counter, h->spec_part, h->spec_out, h->spec_counter, h->stage,
+                  h->sc, h->rb.partials, h->rb.counter, h->stage,
                   h->fft_work};
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -1343,10 +1322,7 @@ int lat_create(lat_t** out, const lat_config* cfg) {
   h->red_cap = maxb;
   if ((st = alloc((void**)&h->rb.partials, (size_t)maxb * 16 * sizeof(double)))) return bail(st);
   if ((st = alloc((void**)&h->rb.counter, 64))) return bail(st);
-  h->spec_grid = h->nsm * 2;
-  if ((st = alloc((void**)&h->spec_part, (size_t)h->spec_grid * 3 * kMaxBins * sizeof(double)))) return bail(st);
-  if ((st = alloc((void**)&h->spec_out, (size_t)3 * kMaxBins * sizeof(double)))) return bail(st);
-  if ((st = alloc((void**)&h->spec_counter, 64))) return bail(st);
+  if ((st = h->bins.make(h->nx, h->ny, h->nz, h->nsm, h->stream))) return bail(st);
   h->fd_ty = 8;
   h->fd_zc = std::min(32, h->nz);
 
@@ -1676,13 +1652,8 @@ int lat_spectrum(lat_t* h, int32_t what, int32_t field, int32_t mode, int32_t nb
   void* F;
   int sp;
   RET(output_spectrum(h, what, field, 0, &F, &sp));
-  std::vector<double> o(3 * nbins);
-  RET(run_spectrum(h, F, nullptr, mode, nbins, o.data(), sp));
-  for (int l = 0; l < nbins; ++l) {
-    W[l] = o[nbins + l];
-    S[l] = W[l] != 0.0 ? o[l] / W[l] : o[l];
-  }
-  return LAT_OK;
+  Timed t(h, LAT_K_OTHER);
+  return h->bins.power(F, mode, sp, nbins, S, W, h->stream);
 }
 
 int lat_crossspec(lat_t* h, int32_t what1, int32_t field1, int32_t what2, int32_t field2, int32_t nbins,
@@ -1695,14 +1666,8 @@ int lat_crossspec(lat_t* h, int32_t what1, int32_t field1, int32_t what2, int32_
   int sp;
   RET(output_spectrum(h, what1, field1, 0, &F1, &sp));
   RET(output_spectrum(h, what2, field2, 1, &F2, &sp));
-  std::vector<double> o(3 * nbins);
-  RET(run_spectrum(h, F1, F2, 2, nbins, o.data(), sp));
-  for (int l = 0; l < nbins; ++l) {
-    const double w = o[nbins + l];
-    S_re[l] = w != 0.0 ? o[l] / w : o[l];
-    S_im[l] = w != 0.0 ? o[2 * nbins + l] / w : o[2 * nbins + l];
-  }
-  return LAT_OK;
+  Timed t(h, LAT_K_OTHER);
+  return h->bins.cross(F1, F2, sp, nbins, S_re, S_im, h->stream);
 }
 
 int lat_gw_spectrum(lat_t* h, int32_t nbins, double* S, double* W) {
@@ -1719,28 +1684,10 @@ int lat_gw_spectrum(lat_t* h, int32_t nbins, double* S, double* W) {
     RET(make_plan(h, &h->p_r2c6, &h->have_r2c6, true, 6));
     RET(fft_exec_r2c(h, h->p_r2c6, h->pu, h->Fk6));
   }
-  GwSpecArgs a{};
-  a.nx = h->nx; a.ny = h->ny; a.nz = h->nz;
-  for (int c = 0; c < 6; ++c) a.F[c] = (const char*)h->Fk6 + (size_t)c * h->M * h->csz;
-  a.dx = h->dx;
-  a.nbins = nbins;
-  a.partials = h->spec_part;
-  a.out = h->spec_out;
-  a.counter = h->spec_counter;
-  a.grid = h->spec_grid;
-  a.block = 256;
-  {
-    Timed t(h, LAT_K_OTHER);
-    RET(launch_gw_spectrum(a, h->prec, h->stream));
-  }
-  std::vector<double> o(2 * nbins);
-  CK(cudaMemcpyAsync(o.data(), h->spec_out, sizeof(double) * 2 * nbins, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
-  for (int l = 0; l < nbins; ++l) {
-    W[l] = o[nbins + l];
-    S[l] = W[l] != 0.0 ? o[l] / W[l] : o[l];
-  }
-  return LAT_OK;
+  const void* F[6];
+  for (int c = 0; c < 6; ++c) F[c] = (const char*)h->Fk6 + (size_t)c * h->M * h->csz;
+  Timed t(h, LAT_K_OTHER);
+  return h->bins.gw(F, h->prec, nbins, S, W, h->stream);
 }
 
 // GW strains and momenta of a z-slab's interior planes, [6][nz_loc][ny][nx].

@@ -273,31 +273,6 @@ int launch_cube(const void* hi, const void* c, int nx, int ny, int nz, int ds, i
                 cudaStream_t s);
 int launch_from_fp64(const double* in, int64_t n, int precision, void* hi, void* c, cudaStream_t s);
 
-struct SpecArgs {
-  int nx, ny, nz;
-  const void* F1;  // half spectrum [z][y][nx/2+1]
-  const void* F2;  // second spectrum for the cross spectrum (nullptr otherwise)
-  int mode;        // LAT_SPEC_WEIGHTED / LAT_SPEC_COUNT / 2 = cross (weighted)
-  int nbins;
-  double* partials;   // [grid][3*nbins]
-  double* out;        // [3*nbins]: S (or S_re), W, S_im
-  unsigned int* counter;
-  int grid, block;
-};
-int launch_spectrum(const SpecArgs& a, int precision, cudaStream_t s);
-
-struct GwSpecArgs {
-  int nx, ny, nz;
-  const void* F[6];
-  double dx;
-  int nbins;
-  double* partials;
-  double* out;  // [2*nbins]
-  unsigned int* counter;
-  int grid, block;
-};
-int launch_gw_spectrum(const GwSpecArgs& a, int precision, cudaStream_t s);
-
 // Energies: raw lattice sums into sc->red:
 // [0] sum pi^2, [1] sum V, [2] sum phi_1, [3] sum phi_2, [4] -sum phi L phi (FD),
 // [5] sum STENCIL(c,GRAD2) (FD), [6] sum pu^2, [7] -sum u L u (GW, weighted)

@@ -22,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "bin.hpp"
 #include "engine.hpp"
 #include "integrator.hpp"
 
@@ -174,6 +175,7 @@ struct lat_ens_s {
     // encoded once: the class's arrays never move
     CUtensorMap tm_zs[2] = {}, tm_pi[2] = {};
     bool tm_ok[2] = {false, false};
+    BinPlan bins;             // spectra of this size
   };
   std::vector<Cls> cls;
   std::vector<int> run_cls;
@@ -184,9 +186,6 @@ struct lat_ens_s {
   size_t work_size = 0;
   DevScalars* sc = nullptr;
   RedBuf rb{};
-  double* spec_part = nullptr;
-  double* spec_out = nullptr;
-  unsigned int* spec_counter = nullptr;
   int grid = 0, block = 256;
   bool sep_ok = false;  // every class can run the streamed separable passes (pairs of runs)
   bool sep = false;     // and they are in use (else cuFFT per class)
@@ -482,10 +481,10 @@ int lat_ens_destroy(lat_ens_t* e) {
     if (c.shift) cudaFree(c.shift);
     if (c.side) cudaStreamDestroy(c.side);
     if (c.done) cudaEventDestroy(c.done);
+    c.bins.free();
   }
   if (e->fork) cudaEventDestroy(e->fork);
-  void* bufs[] = {e->phi, e->phic, e->pi, e->lap, e->Fk, e->work, e->sc, e->rb.partials, e->rb.counter,
-                  e->spec_part, e->spec_out, e->spec_counter};
+  void* bufs[] = {e->phi, e->phic, e->pi, e->lap, e->Fk, e->work, e->sc, e->rb.partials, e->rb.counter};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (e->stream) cudaStreamDestroy(e->stream);
@@ -567,9 +566,6 @@ int lat_ens_create(lat_ens_t** out, const lat_config* base, int32_t nruns, const
   if ((st = alloc((void**)&e->sc, sizeof(DevScalars)))) return bail(st);
   if ((st = alloc((void**)&e->rb.partials, (size_t)8192 * 16 * sizeof(double)))) return bail(st);
   if ((st = alloc((void**)&e->rb.counter, 64))) return bail(st);
-  if ((st = alloc((void**)&e->spec_part, (size_t)e->nsm * 2 * 3 * 2048 * sizeof(double)))) return bail(st);
-  if ((st = alloc((void**)&e->spec_out, (size_t)3 * 2048 * sizeof(double)))) return bail(st);
-  if ((st = alloc((void**)&e->spec_counter, 64))) return bail(st);
   const bool d = e->prec == LAT_FP64;
   for (auto& c : e->cls) {
     if ((st = plan(e, &c.r2c, c.n, c.count, d ? CUFFT_D2Z : CUFFT_R2C))) return bail(st);
@@ -577,6 +573,7 @@ int lat_ens_create(lat_ens_t** out, const lat_config* base, int32_t nruns, const
     if ((st = plan(e, &c.r2c1, c.n, 1, d ? CUFFT_D2Z : CUFFT_R2C))) return bail(st);
     if ((st = plan(e, &c.z2d1, c.n, 1, CUFFT_Z2D))) return bail(st);
     c.have = true;
+    if ((st = c.bins.make(c.n, c.n, c.n, e->nsm, e->stream))) return bail(st);
   }
   // the streamed separable passes: FP32, every class of a supported side with
   // an even run count, every pass in whole tiles (LAT_ENS_CUFFT=1: cuFFT)
@@ -908,7 +905,7 @@ int lat_ens_energies(lat_ens_t* e, double* out) {
 }
 
 int lat_ens_spectrum(lat_ens_t* e, int32_t run, int32_t nbins, double* S, double* W) {
-  if (!e || !S || !W || nbins < 1 || nbins > 2048) return set_error(LAT_ERR_ARG, "bad spectrum arguments");
+  if (!e || !S || !W || nbins < 1 || nbins > kMaxBins) return set_error(LAT_ERR_ARG, "bad spectrum arguments");
   EGuard g(e);
   char *f, *c, *p;
   const lat_ens_s::Cls* cl;
@@ -916,25 +913,7 @@ int lat_ens_spectrum(lat_ens_t* e, int32_t run, int32_t nbins, double* S, double
   cufftResult fr = e->prec == LAT_FP64 ? cufftExecD2Z(cl->r2c1, (cufftDoubleReal*)f, (cufftDoubleComplex*)e->Fk)
                                        : cufftExecR2C(cl->r2c1, (cufftReal*)f, (cufftComplex*)e->Fk);
   if (fr != CUFFT_SUCCESS) return set_error(LAT_ERR_CUDA, "ensemble spectrum FFT");
-  SpecArgs sa{};
-  sa.nx = sa.ny = sa.nz = cl->n;
-  sa.F1 = e->Fk;
-  sa.mode = LAT_SPEC_WEIGHTED;
-  sa.nbins = nbins;
-  sa.partials = e->spec_part;
-  sa.out = e->spec_out;
-  sa.counter = e->spec_counter;
-  sa.grid = e->nsm * 2;
-  sa.block = 256;
-  ERET(launch_spectrum(sa, e->prec, e->stream));
-  std::vector<double> o(3 * nbins);
-  ECK(cudaMemcpyAsync(o.data(), e->spec_out, sizeof(double) * 3 * nbins, cudaMemcpyDeviceToHost, e->stream));
-  ECK(cudaStreamSynchronize(e->stream));
-  for (int l = 0; l < nbins; ++l) {
-    W[l] = o[nbins + l];
-    S[l] = W[l] != 0.0 ? o[l] / W[l] : o[l];
-  }
-  return LAT_OK;
+  return e->cls[e->run_cls[run]].bins.power(e->Fk, LAT_SPEC_WEIGHTED, e->prec, nbins, S, W, e->stream);
 }
 
 int lat_ens_download(lat_ens_t* e, int32_t run, double* fld, double* fldp) {

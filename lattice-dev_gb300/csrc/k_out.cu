@@ -1,4 +1,4 @@
-// k_out.cu -- layout conversion, spectra, energies and initial conditions.
+// k_out.cu -- layout conversion, energies and initial conditions.
 #include "engine.hpp"
 
 namespace lat {
@@ -58,159 +58,6 @@ inline int done(const char* what) {
   if (g_launch_counter) ++*g_launch_counter;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? LAT_OK : cuda_fail(e, what);
-}
-
-// ------------------------------------------------------------ spectra
-// Array grid reduction: every block adds its shared bins to partials[block],
-// the last block sums the rows in block order.
-__device__ void bins_grid_reduce(const double* shb, int nval, double* partials, double* out,
-                                 unsigned int* counter) {
-  __shared__ int am_last;
-  const int bid = blockIdx.x;
-  for (int i = threadIdx.x; i < nval; i += blockDim.x) partials[(size_t)bid * nval + i] = shb[i];
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int t = atomicAdd(counter, 1u);
-    am_last = (t == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!am_last) return;
-  __threadfence();
-  for (int i = threadIdx.x; i < nval; i += blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < (int)gridDim.x; ++b) s += __ldcg(&partials[(size_t)b * nval + i]);
-    out[i] = s;
-  }
-  if (threadIdx.x == 0) *counter = 0u;
-}
-
-// Binning of spectrum_3d (analysis_spec.f90:86-99) / spectrum_bin
-// (Discrete/Bubble-Collisions/analysis.f90:203-214).  The reference loops over
-// the full x range with folded ii, i.e. Hermitian weight 2 on interior kx
-// planes.  Shell index l = floor(sqrt(ii^2+jj^2+kk^2)) is taken exactly in
-// integers; the smooth weights use the correctly rounded FP64 sqrt and
-// uncontracted FP64 arithmetic so they are bit-identical to the host's.
-template <typename R, typename C>
-__global__ void __launch_bounds__(256) spec_kernel(SpecArgs a) {
-  extern __shared__ double shb[];  // [3][nbins]
-  const int nb = a.nbins;
-  for (int i = threadIdx.x; i < 3 * nb; i += blockDim.x) shb[i] = 0.0;
-  __syncthreads();
-  const C* F1 = static_cast<const C*>(a.F1);
-  const C* F2 = static_cast<const C*>(a.F2);
-  const unsigned int hx = a.nx / 2 + 1, ny = a.ny;
-  const unsigned int M = hx * ny * (unsigned int)a.nz;
-  for (unsigned int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-    const int x = (int)(m % hx);
-    const unsigned int r = m / hx;
-    const int y = (int)(r % ny), z = (int)(r / ny);
-    const int jj = fold_idx(y, a.ny), kk = fold_idx(z, a.nz);
-    const double wx = (x == 0 || 2 * x == a.nx) ? 1.0 : 2.0;
-    const int m2 = x * x + jj * jj + kk * kk;
-    const int l = isqrt_exact(m2);
-    const C f1 = F1[m];
-    double v, vi = 0.0;
-    if (a.mode == 2) {
-      const C f2 = F2[m];
-      v = (double)f1.x * (double)f2.x + (double)f1.y * (double)f2.y;   // Re(F1 conj F2)
-      vi = (double)f1.y * (double)f2.x - (double)f1.x * (double)f2.y;  // Im(F1 conj F2)
-    } else {
-      v = (double)f1.x * (double)f1.x + (double)f1.y * (double)f1.y;
-    }
-    if (a.mode == LAT_SPEC_COUNT) {
-      if (l < nb) {
-        atomicAdd(&shb[l], wx * v);
-        atomicAdd(&shb[nb + l], wx);
-      }
-    } else {
-      const double p = sqrt((double)m2);
-      const double d0 = __dsub_rn((double)l, p), d1 = __dsub_rn((double)(l + 1), p);
-      const double e0 = __dsub_rn(1.0, __dmul_rn(d0, d0)), e1 = __dsub_rn(1.0, __dmul_rn(d1, d1));
-      const double c0 = __dmul_rn(e0, e0), c1 = __dmul_rn(e1, e1);
-      if (l < nb) {
-        atomicAdd(&shb[l], wx * c0 * v);
-        atomicAdd(&shb[nb + l], wx * c0);
-        if (a.mode == 2) atomicAdd(&shb[2 * nb + l], wx * c0 * vi);
-      }
-      if (l + 1 < nb) {
-        atomicAdd(&shb[l + 1], wx * c1 * v);
-        atomicAdd(&shb[nb + l + 1], wx * c1);
-        if (a.mode == 2) atomicAdd(&shb[2 * nb + l + 1], wx * c1 * vi);
-      }
-    }
-  }
-  __syncthreads();
-  bins_grid_reduce(shb, 3 * nb, a.partials, a.out, a.counter);
-}
-
-// TT projection of the six pi_ij with the lattice momentum of the central
-// difference, k_i = sin(2 pi n_i / N_i)/dx:  P = 1 - k k^T/k^2,
-// pi^TT = P pi P - P tr(P pi)/2;  sum_ij |pi^TT_ij|^2 binned like spectrum_bin.
-template <typename R, typename C>
-__global__ void __launch_bounds__(256) gwspec_kernel(GwSpecArgs a) {
-  extern __shared__ double shb[];  // [2][nbins]
-  const int nb = a.nbins;
-  for (int i = threadIdx.x; i < 2 * nb; i += blockDim.x) shb[i] = 0.0;
-  __syncthreads();
-  const unsigned int hx = a.nx / 2 + 1, ny = a.ny;
-  const unsigned int M = hx * ny * (unsigned int)a.nz;
-  const double twopi = 6.283185307179586476925286766559;
-  for (unsigned int m = blockIdx.x * blockDim.x + threadIdx.x; m < M; m += gridDim.x * blockDim.x) {
-    const int x = (int)(m % hx);
-    const unsigned int r = m / hx;
-    const int y = (int)(r % ny), z = (int)(r / ny);
-    const int jj = fold_idx(y, a.ny), kk = fold_idx(z, a.nz);
-    const double wx = (x == 0 || 2 * x == a.nx) ? 1.0 : 2.0;
-    const int l = isqrt_exact(x * x + jj * jj + kk * kk);
-    if (l >= nb) continue;
-    double k[3] = {sin(twopi * x / a.nx) / a.dx, sin(twopi * y / a.ny) / a.dx, sin(twopi * z / a.nz) / a.dx};
-    const double k2 = k[0] * k[0] + k[1] * k[1] + k[2] * k[2];
-    double sum = 0.0;
-    if (k2 > 0.0) {
-      double P[3][3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) P[i][j] = (i == j ? 1.0 : 0.0) - k[i] * k[j] / k2;
-      const int map[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
-      double hr[3][3], hi[3][3];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          const C v = static_cast<const C*>(a.F[map[i][j]])[m];
-          hr[i][j] = (double)v.x;
-          hi[i][j] = (double)v.y;
-        }
-      double Ar[3][3], Ai[3][3];  // A = P h
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          double sr = 0, si = 0;
-#pragma unroll
-          for (int l2 = 0; l2 < 3; ++l2) { sr += P[i][l2] * hr[l2][j]; si += P[i][l2] * hi[l2][j]; }
-          Ar[i][j] = sr; Ai[i][j] = si;
-        }
-      double trr = Ar[0][0] + Ar[1][1] + Ar[2][2], tri = Ai[0][0] + Ai[1][1] + Ai[2][2];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          double sr = 0, si = 0;
-#pragma unroll
-          for (int l2 = 0; l2 < 3; ++l2) { sr += Ar[i][l2] * P[l2][j]; si += Ai[i][l2] * P[l2][j]; }
-          sr -= 0.5 * P[i][j] * trr;
-          si -= 0.5 * P[i][j] * tri;
-          sum += sr * sr + si * si;
-        }
-    }
-    atomicAdd(&shb[l], wx * sum);
-    atomicAdd(&shb[nb + l], wx);
-  }
-  __syncthreads();
-  bins_grid_reduce(shb, 2 * nb, a.partials, a.out, a.counter);
 }
 
 // ------------------------------------------------------------ energies
@@ -625,20 +472,6 @@ int launch_from_fp64(const double* in, int64_t n, int precision, void* hi, void*
   if (precision == LAT_FP64) from64_kernel<double, false><<<grid_for(n), 256, 0, s>>>(in, n, (double*)hi, nullptr);
   else from64_kernel<float, true><<<grid_for(n), 256, 0, s>>>(in, n, (float*)hi, (float*)c);
   return done("from_fp64");
-}
-
-int launch_spectrum(const SpecArgs& a, int precision, cudaStream_t s) {
-  const size_t smem = (size_t)3 * a.nbins * sizeof(double);
-  if (precision == LAT_FP64) spec_kernel<double, double2><<<a.grid, a.block, smem, s>>>(a);
-  else spec_kernel<float, float2><<<a.grid, a.block, smem, s>>>(a);
-  return done("spectrum");
-}
-
-int launch_gw_spectrum(const GwSpecArgs& a, int precision, cudaStream_t s) {
-  const size_t smem = (size_t)2 * a.nbins * sizeof(double);
-  if (precision == LAT_FP64) gwspec_kernel<double, double2><<<a.grid, a.block, smem, s>>>(a);
-  else gwspec_kernel<float, float2><<<a.grid, a.block, smem, s>>>(a);
-  return done("gw spectrum");
 }
 
 int launch_energy(const EnergyArgs& a, int precision, cudaStream_t s) {
