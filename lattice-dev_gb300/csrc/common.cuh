@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../../include/lattice.h"
 
 namespace lat {
@@ -144,6 +146,75 @@ template <typename R> struct AccOf;
 template <> struct AccOf<float> { using type = KSum; };
 template <> struct AccOf<double> { using type = DSum; };
 
+// Block sums of NV values per thread into sum[i], valid in every thread after
+// the closing barrier.  A warp-wide FP64 addition holds GB300's FP64 pipe for
+// 16 clocks, so up to four doubles per thread are added through shared memory
+// (one warp per value: nthreads / 32 + 5 additions) instead of five shuffles
+// per warp and value; float-float values take the shuffles, whose additions
+// are FP32.  At most 512 threads.
+template <int NV, typename T>
+__device__ __forceinline__ void block_sums(const T (&v)[NV], double (&sum)[NV]) {
+  const int nthreads = blockDim.x * blockDim.y * blockDim.z;
+  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  const int lane = tid & 31, wid = tid >> 5, nw = (nthreads + 31) >> 5;
+  if constexpr (sizeof(T) == sizeof(double) && NV <= 4 && !std::is_same<T, FF>::value) {
+    __shared__ double st[NV][512];
+    __shared__ double tot[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) st[i][tid] = v[i];
+    __syncthreads();
+    for (int i = wid; i < NV; i += nw) {
+      double x = 0.0;
+      for (int k = lane; k < nthreads; k += 32) x += st[i][k];
+      x = warp_sum(x);
+      if (lane == 0) tot[i] = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NV; ++i) sum[i] = tot[i];
+  } else {
+    __shared__ double sh[NV][17];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const double x = warp_sum(v[i]);
+      if (lane == 0) sh[i][wid] = x;
+    }
+    __syncthreads();
+    for (int i = wid; i < NV; i += nw) {
+      const double x = warp_sum(lane < nw ? sh[i][lane] : 0.0);
+      __syncwarp();
+      if (lane == 0) sh[i][16] = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < NV; ++i) sum[i] = sh[i][16];
+  }
+}
+
+// Sums of NV values over the rows part[b][NV], b < nblk, one warp per value;
+// valid in every thread.  The order is fixed.
+template <int NV>
+__device__ __forceinline__ void row_sums(const double* part, int nblk, double (&total)[NV]) {
+  __shared__ double tot[NV];
+  const int nthreads = blockDim.x * blockDim.y * blockDim.z;
+  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  const int lane = tid & 31, wid = tid >> 5, nw = (nthreads + 31) >> 5;
+  for (int i = wid; i < NV; i += nw) {
+    double x[4] = {0.0, 0.0, 0.0, 0.0};
+    int b = lane;
+    for (; b + 96 < nblk; b += 128) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] += __ldcg(part + (size_t)(b + 32 * k) * NV + i);
+    }
+    for (; b < nblk; b += 32) x[0] += __ldcg(part + (size_t)b * NV + i);
+    const double y = warp_sum((x[0] + x[1]) + (x[2] + x[3]));
+    if (lane == 0) tot[i] = y;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < NV; ++i) total[i] = tot[i];
+}
+
 // Deterministic grid reduction of NV values (doubles, or float-float warp
 // inputs): block partials are written in block order and the last block to
 // arrive sums them in a fixed order, so two identical launches give
@@ -152,53 +223,24 @@ template <> struct AccOf<double> { using type = DSum; };
 // reuse it).  All threads of every block must call it.
 template <int NV, typename T>
 __device__ __forceinline__ bool grid_reduce(const T (&v)[NV], const RedBuf rb, double (&total)[NV]) {
-  __shared__ double sh[NV][32];
   __shared__ int am_last;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int nthreads = blockDim.x * blockDim.y * blockDim.z;
   const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
-  const int lane2 = tid & 31, wid2 = tid >> 5, nw = (nthreads + 31) >> 5;
-  (void)lane; (void)wid;
   const int bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
   const int nblk = gridDim.x * gridDim.y * gridDim.z;
+  double s[NV];
+  block_sums<NV>(v, s);
+  if (tid == 0) {
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    double x = warp_sum(v[i]);
-    if (lane2 == 0) sh[i][wid2] = x;
-  }
-  __syncthreads();
-  if (wid2 == 0) {
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      double x = lane2 < nw ? sh[i][lane2] : 0.0;
-      x = warp_sum(x);
-      if (lane2 == 0) rb.partials[(size_t)bid * NV + i] = x;
-    }
-    if (lane2 == 0) {
-      __threadfence();
-      unsigned int t = atomicAdd(rb.counter, 1u);
-      am_last = (t == (unsigned int)nblk - 1u);
-    }
+    for (int i = 0; i < NV; ++i) rb.partials[(size_t)bid * NV + i] = s[i];
+    __threadfence();
+    const unsigned int t = atomicAdd(rb.counter, 1u);
+    am_last = (t == (unsigned int)nblk - 1u);
   }
   __syncthreads();
   if (!am_last) return false;
   __threadfence();
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    double x = 0.0;
-    for (int b = tid; b < nblk; b += nthreads) x += __ldcg(&rb.partials[(size_t)b * NV + i]);
-    x = warp_sum(x);
-    __syncthreads();
-    if (lane2 == 0) sh[i][wid2] = x;
-  }
-  __syncthreads();
+  row_sums<NV>(rb.partials, nblk, total);
   if (tid != 0) return false;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += sh[i][w];
-    total[i] = s;
-  }
   *rb.counter = 0u;
   return true;
 }
@@ -228,18 +270,25 @@ __device__ __forceinline__ void block_partials(const T (&v)[NV], double* out) {
 __device__ __forceinline__ bool bad(double x) { return !(x - x == 0.0); }
 
 // ---------------------------------------------------------------- models
-// potential / modeldv of the reference models (V, not DEFROST's 2V).
+// potential / modeldv of the reference models (V, not DEFROST's 2V).  In FP64
+// the products are arranged for the fewest operations (7 instead of 9 for the
+// coupled force, 5 instead of 9 for its potential): the FP64 pipe bounds every
+// pass that evaluates them.
 template <typename R, int NF>
 __device__ __forceinline__ void model_dv(const ModelP& m, const R (&f)[NF], R (&dv)[NF]) {
   const R p0 = (R)m.p[0], p1 = (R)m.p[1];
   switch (m.model) {
     case LAT_MODEL_PHI4:
-      dv[0] = p0 * f[0] * f[0] * f[0];
+      dv[0] = sizeof(R) == 8 ? p0 * (f[0] * f[0]) * f[0] : p0 * f[0] * f[0] * f[0];
 #pragma unroll
       for (int l = 1; l < NF; ++l) dv[l] = R(0);
       break;
     case LAT_MODEL_PHI4_G2:
-      if constexpr (NF >= 2) {
+      if constexpr (NF >= 2 && sizeof(R) == 8) {
+        const R x2 = f[0] * f[0], y2 = f[1] * f[1];
+        dv[0] = f[0] * fma(p1, y2, p0 * x2);
+        dv[1] = (p1 * x2) * f[1];
+      } else if constexpr (NF >= 2) {
         dv[0] = p0 * f[0] * f[0] * f[0] + p1 * f[0] * f[1] * f[1];
         dv[1] = p1 * f[0] * f[0] * f[1];
       } else {
@@ -261,9 +310,17 @@ template <typename R, int NF>
 __device__ __forceinline__ R model_v(const ModelP& m, const R (&f)[NF]) {
   const R p0 = (R)m.p[0], p1 = (R)m.p[1];
   switch (m.model) {
-    case LAT_MODEL_PHI4: return R(0.25) * p0 * f[0] * f[0] * f[0] * f[0];
+    case LAT_MODEL_PHI4:
+      if constexpr (sizeof(R) == 8) {
+        const R x2 = f[0] * f[0];
+        return (R(0.25) * p0) * (x2 * x2);
+      }
+      return R(0.25) * p0 * f[0] * f[0] * f[0] * f[0];
     case LAT_MODEL_PHI4_G2:
-      if constexpr (NF >= 2)
+      if constexpr (NF >= 2 && sizeof(R) == 8) {
+        const R x2 = f[0] * f[0], y2 = f[1] * f[1];
+        return x2 * fma(R(0.5) * p1, y2, (R(0.25) * p0) * x2);
+      } else if constexpr (NF >= 2)
         return R(0.25) * p0 * f[0] * f[0] * f[0] * f[0] + R(0.5) * p1 * f[0] * f[0] * f[1] * f[1];
       else
         return R(0.25) * p0 * f[0] * f[0] * f[0] * f[0];

@@ -301,6 +301,25 @@ int launch_parseval(const void* Fk, int nx, int ny, int nz, int nf, double dkx2,
                     double dkz2, DevScalars* sc, int slot, RedBuf rb, int grid, int precision,
                     cudaStream_t s);
 
+// Energies of every run of an ensemble (k_energy.cu)
+struct EnsEnergyRun {
+  int64_t site, fk;  // the run's first site and first mode (elements)
+  double dk2;
+  int n, blocks;     // side; blocks of the launch that share the run
+};
+struct EnsEnergyArgs {
+  const EnsEnergyRun* runs;  // device, one per run
+  const void* phi;
+  const void* pi;
+  const void* Fk;
+  ModelP model;
+  double* partials;          // [run][max_blocks][<= 4]
+  double* out;               // [run][8]: sum pi^2, V, phi; [4] Parseval sum
+  unsigned int* counters;    // one per run, left at zero
+  int max_blocks;
+};
+int launch_ens_energies(const EnsEnergyArgs& a, int nruns, int parseval, int precision, cudaStream_t s);
+
 struct VacArgs {
   int nx, ny, nz;
   uint64_t seed;

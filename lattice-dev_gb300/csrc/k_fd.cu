@@ -637,7 +637,7 @@ int go2(const FdArgs& a, cudaStream_t s, int* nb) {
   dim3 grid(a.nx / 64, (a.ny + a.ty - 1) / a.ty, (nzc + a.zc - 1) / a.zc);
   const size_t smem = (size_t)3 * NC * kFd2Wd * (a.ty + 2) * sizeof(float);
   auto k = fd2_kernel<KAHAN, NF, GW, SEVEN, MODE>;
-  if (smem > 48 * 1024) {
+  if (smem > 30 * 1024) {  // the reduction's static arrays count towards the 48 KB too
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "fd2 smem attribute");
   }
@@ -663,7 +663,7 @@ int go(const FdArgs& a0, cudaStream_t s, int* nb) {
   if (a.ty < 1 || (!a.vec && 34 * (a.ty + 2) > kFdMaxSlots * 32 * a.ty))
     return set_error(LAT_ERR_ARG, "FD tile too narrow");
   auto k = fd_kernel<R, KAHAN, NF, GW, SEVEN, MODE>;
-  if (smem > 48 * 1024) {
+  if (smem > 30 * 1024) {  // the reduction's static arrays count towards the 48 KB too
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "fd smem attribute");
   }

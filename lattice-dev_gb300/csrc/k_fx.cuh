@@ -396,10 +396,9 @@ template <int NF, int AXIS, int N, bool CONF>
 int fx_go(const SepArgs& a, cudaStream_t s) {
   using G = Geo<N>;
   auto k = fx_kernel<NF, AXIS, N, CONF>;
-  if (G::SMEM > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-    if (e != cudaSuccess) return cuda_fail(e, "fixed-point pass smem attribute");
-  }
+  // also below 48 KB, which the static arrays count towards
+  const cudaError_t ea = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
+  if (ea != cudaSuccess) return cuda_fail(ea, "fixed-point pass smem attribute");
   const int64_t tiles = a.nlines / kLines;
   if (a.nlines % kLines) return set_error(LAT_ERR_STATE, "fixed-point pass: partial tile");
   const int grid = (int)std::min<int64_t>(tiles, (int64_t)a.nsm * G::MINB);

@@ -1,4 +1,4 @@
-// k_out.cu -- layout conversion, energies and initial conditions.
+// k_out.cu -- layout conversion and initial conditions.
 #include "engine.hpp"
 
 namespace lat {
@@ -58,167 +58,6 @@ inline int done(const char* what) {
   if (g_launch_counter) ++*g_launch_counter;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? LAT_OK : cuda_fail(e, what);
-}
-
-// ------------------------------------------------------------ energies
-template <typename R, bool KAHAN, int NF>
-__global__ void __launch_bounds__(256) energy_kernel(EnergyArgs a) {
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const int64_t N = (int64_t)nx * ny * nz;
-  const R* phi = static_cast<const R*>(a.phi);
-  const R* pi = static_cast<const R*>(a.pi);
-  const R* u = static_cast<const R*>(a.u);
-  const R* pu = static_cast<const R*>(a.pu);
-  using Acc = typename AccOf<R>::type;
-  Acc s[11];
-  const R c0 = (R)a.c[0], c1 = (R)a.c[1], c2 = (R)a.c[2], c3 = (R)a.c[3];
-  int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool ranged = a.t_hi > 0;  // a z-slab: only its interior sites
-  const int64_t tend = ranged ? a.t_hi : N;
-  if (ranged) t0 += a.t_lo;
-  if constexpr (sizeof(R) == 4) {
-    // spectral, no GW arrays: four sites per thread and step (float4 loads),
-    // one compensated add per sum and four sites
-    if (!ranged && !a.fd && !u && N % 4 == 0) {  // every field's array starts 16-byte aligned
-      const int64_t n4 = N / 4;
-      for (int64_t v = t0; v < n4; v += (int64_t)gridDim.x * blockDim.x) {
-        float4 fq[NF], pq[NF];
-#pragma unroll
-        for (int l = 0; l < NF; ++l) {
-          fq[l] = __ldcs(reinterpret_cast<const float4*>(phi + l * N) + v);
-          pq[l] = __ldcs(reinterpret_cast<const float4*>(pi + l * N) + v);
-        }
-        R ke = 0, pe = 0, m0 = 0, m1 = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          R f[NF];
-#pragma unroll
-          for (int l = 0; l < NF; ++l) {
-            const float4 F4 = fq[l], P4 = pq[l];
-            f[l] = j == 0 ? F4.x : (j == 1 ? F4.y : (j == 2 ? F4.z : F4.w));
-            const R p = j == 0 ? P4.x : (j == 1 ? P4.y : (j == 2 ? P4.z : P4.w));
-            ke += p * p;
-          }
-          pe += model_v<R, NF>(a.model, f);
-          m0 += f[0];
-          if (NF > 1) m1 += f[NF > 1 ? 1 : 0];
-        }
-        s[0].add(ke);
-        s[1].add(pe);
-        s[2].add(m0);
-        if (NF > 1) s[3].add(m1);
-      }
-      t0 = N;  // no tail
-    }
-  }
-  for (int64_t t = t0; t < tend; t += (int64_t)gridDim.x * blockDim.x) {
-    R f[NF];
-#pragma unroll
-    for (int l = 0; l < NF; ++l) {
-      f[l] = phi[l * N + t];
-      const R p = pi[l * N + t];
-      s[0].add(p * p);
-    }
-    s[1].add(model_v<R, NF>(a.model, f));
-    s[2].add(f[0]);
-    if (NF > 1) s[3].add(f[NF > 1 ? 1 : 0]);
-    if (a.fd || u) {
-      const int x = (int)(t % nx), y = (int)((t / nx) % ny), z = (int)(t / ((int64_t)nx * ny));
-      auto wrapi = [](int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); };
-      auto stencil = [&](const R* g, R& lapsum, R& grad2) {
-        const R g0 = g[t];
-        R r1 = 0, r2 = 0, r3 = 0, q1 = 0, q2 = 0, q3 = 0;
-        for (int dz = -1; dz <= 1; ++dz)
-          for (int dy = -1; dy <= 1; ++dy)
-            for (int dx = -1; dx <= 1; ++dx) {
-              const int rank = (dx != 0) + (dy != 0) + (dz != 0);
-              if (rank == 0) continue;
-              const R v = g[((int64_t)wrapi(z + dz, nz) * ny + wrapi(y + dy, ny)) * nx + wrapi(x + dx, nx)];
-              const R d = v - g0;
-              if (rank == 1) { r1 += v; q1 += d * d; }
-              else if (rank == 2) { r2 += v; q2 += d * d; }
-              else { r3 += v; q3 += d * d; }
-            }
-        lapsum = c0 * g0 + c1 * r1 + c2 * r2 + c3 * r3;
-        grad2 = c1 * q1 + c2 * q2 + c3 * q3;
-      };
-      if (a.fd) {
-        R g2sum = 0;
-#pragma unroll
-        for (int l = 0; l < NF; ++l) {
-          R ls, g2;
-          stencil(phi + l * N, ls, g2);
-          s[4].add(-f[l] * ls);
-          s[5].add(g2);
-          g2sum += g2;
-        }
-        if (a.ball_r2 > 0.0) {  // 1-based indices about n/2 (iofile.f90:552)
-          const double bx = x + 1 - nx / 2, by = y + 1 - ny / 2, bz = z + 1 - nz / 2;
-          if ((bx * bx + by * by + bz * bz) * a.dx * a.dx < a.ball_r2) {
-            R psum = 0;
-#pragma unroll
-            for (int l = 0; l < NF; ++l) psum += pi[l * N + t];
-            s[8].add(psum * psum);
-            s[9].add(g2sum);
-            s[10].add(model_v<R, NF>(a.model, f));
-          }
-        }
-      }
-      if (u) {
-        for (int g = 0; g < 6; ++g) {
-          const R w = g < 3 ? R(1) : R(2);
-          const R p = pu[g * N + t];
-          s[6].add(w * p * p);
-          R ls, g2;
-          stencil(u + g * N, ls, g2);
-          s[7].add(-w * u[g * N + t] * ls);
-        }
-      }
-    }
-  }
-  typename Acc::Red v[11];
-  double tot[11];
-#pragma unroll
-  for (int i = 0; i < 11; ++i) v[i] = s[i].red();
-  if (grid_reduce<11>(v, a.rb, tot)) {
-    for (int i = 0; i < 11; ++i) {
-      a.sc->red[i < 8 ? i : i + 1] = tot[i];  // red[8] is the spectral Parseval sum
-      if (bad(tot[i])) a.sc->err |= 1u;
-    }
-  }
-}
-
-// sum over the half spectra of all fields of w k^2 |F_k|^2 (w = 2 for the
-// modes whose conjugate partner is not stored): one warp per row (y, z,
-// field) of nx/2+1 modes, the row's y and z part of k^2 computed once, the
-// terms in the field precision, compensated sums per lane.
-template <typename R, typename C>
-__global__ void __launch_bounds__(256) parseval_kernel(const C* F, int nx, int ny, int nz, int nf, double dkx2,
-                                                       double dky2, double dkz2, DevScalars* sc, int slot,
-                                                       RedBuf rb) {
-  const int hx = nx / 2 + 1;
-  const int64_t rows = (int64_t)ny * nz * nf;
-  const int lane = threadIdx.x & 31;
-  const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  using Acc = typename AccOf<R>::type;
-  Acc acc;
-  for (int64_t row = warp0; row < rows; row += nwarps) {
-    const int64_t rr = row % ((int64_t)ny * nz);
-    const int y = (int)(rr % ny), z = (int)(rr / ny);
-    const int jj = fold_idx(y, ny), kk = fold_idx(z, nz);
-    const R kyz = (R)((double)(jj * jj) * dky2 + (double)(kk * kk) * dkz2);
-    const C* Fr = F + row * hx;
-    for (int x = lane; x < hx; x += 32) {
-      const C v = Fr[x];
-      const R w = (x == 0 || 2 * x == nx) ? R(1) : R(2);
-      const R k2 = (R)(x * x) * (R)dkx2 + kyz;
-      acc.add(w * k2 * (v.x * v.x + v.y * v.y));
-    }
-  }
-  const typename Acc::Red vv[1] = {acc.red()};
-  double t[1];
-  if (grid_reduce<1>(vv, rb, t)) sc->red[slot] = t[0];
 }
 
 // -------------------------------------------------- initial conditions
@@ -472,28 +311,6 @@ int launch_from_fp64(const double* in, int64_t n, int precision, void* hi, void*
   if (precision == LAT_FP64) from64_kernel<double, false><<<grid_for(n), 256, 0, s>>>(in, n, (double*)hi, nullptr);
   else from64_kernel<float, true><<<grid_for(n), 256, 0, s>>>(in, n, (float*)hi, (float*)c);
   return done("from_fp64");
-}
-
-int launch_energy(const EnergyArgs& a, int precision, cudaStream_t s) {
-  if (a.nf == 1) {
-    if (precision == LAT_FP64) energy_kernel<double, false, 1><<<a.grid, a.block, 0, s>>>(a);
-    else energy_kernel<float, true, 1><<<a.grid, a.block, 0, s>>>(a);
-  } else if (a.nf == 2) {
-    if (precision == LAT_FP64) energy_kernel<double, false, 2><<<a.grid, a.block, 0, s>>>(a);
-    else energy_kernel<float, true, 2><<<a.grid, a.block, 0, s>>>(a);
-  } else {
-    return set_error(LAT_ERR_UNSUPPORTED, "energies support nfld = 1 or 2");
-  }
-  return done("energy");
-}
-
-int launch_parseval(const void* Fk, int nx, int ny, int nz, int nf, double dkx2, double dky2, double dkz2,
-                    DevScalars* sc, int slot, RedBuf rb, int grid, int precision, cudaStream_t s) {
-  if (precision == LAT_FP64)
-    parseval_kernel<double, double2><<<grid, 256, 0, s>>>((const double2*)Fk, nx, ny, nz, nf, dkx2, dky2, dkz2, sc, slot, rb);
-  else
-    parseval_kernel<float, float2><<<grid, 256, 0, s>>>((const float2*)Fk, nx, ny, nz, nf, dkx2, dky2, dkz2, sc, slot, rb);
-  return done("parseval");
 }
 
 int launch_vacuum_modes(const VacArgs& a, cudaStream_t s) {
