@@ -241,9 +241,10 @@ bool fx_side(int n) { return n >= 16 && n <= 512 && (n & (n - 1)) == 0; }
 
 // Whether an AUTO lattice takes the separable passes before any autotuning:
 // FP64 lattices that the fixed-point passes tile.  A Yoshida-4 step of two
-// expanding fields: 0.12 ms against 0.24 ms on cuFFT at 32^3, 4.8 against 24.8
+// expanding fields: 0.11 ms against 0.24 ms on cuFFT at 32^3, 4.7 against 24.8
 // at 256^3.  One-field lattices with rows of one tile (32 sites) keep cuFFT,
-// which AUTO has always reported for them.
+// which AUTO has always reported for them; so do FP32 lattices, whose passes
+// round their fields differently (lat_autotune or SEPARABLE choose them).
 bool auto_separable(const lat_s* h) {
   return h->fx_ok && (h->nf == 2 || h->nx >= 64) && !getenv_flag("LAT_NO_SEPARABLE");
 }
@@ -1376,7 +1377,6 @@ int lat_create(lat_t** out, const lat_config* cfg) {
     h->fx_ok = h->prec == LAT_FP64 && fx_side(h->nx) && fx_side(h->ny) && fx_side(h->nz) &&
                h->nx % (h->nf == 2 ? 16 : 32) == 0;
     h->sep = h->sep_ok && cfg->spectral_impl == LAT_SPEC_IMPL_SEPARABLE && !getenv_flag("LAT_NO_SEPARABLE");
-    if (cfg->spectral_impl == LAT_SPEC_IMPL_AUTO) h->sep = auto_separable(h);
     // two FP32 fields on lines of 128 or 256 points whose passes all form
     // whole tiles: the streamed passes (LAT_SEP_CLASSIC=1 keeps the others)
     auto stream_lines = [](int n, int axis) {
@@ -1386,6 +1386,7 @@ int lat_create(lat_t** out, const lat_config* cfg) {
     h->sep_stream = h->sep_ok && h->prec == LAT_FP32_KAHAN && h->nf == 2 && lx && ly && lz &&
                     ((int64_t)h->ny * h->nz) % lx == 0 && h->nx % ly == 0 && h->nx % lz == 0 &&
                     !getenv_flag("LAT_SEP_CLASSIC");
+    if (cfg->spectral_impl == LAT_SPEC_IMPL_AUTO) h->sep = auto_separable(h);
     if (h->sep_ok && h->prec != LAT_FP64) {
       if ((st = alloc(&h->fld[1], fb))) return bail(st);
       if (h->prec == LAT_FP32_KAHAN && (st = alloc(&h->fldc_alt, fb))) return bail(st);

@@ -570,13 +570,13 @@ int lat_ens_create(lat_ens_t** out, const lat_config* base, int32_t nruns, const
   if ((st = alloc((void**)&e->rb.partials, (size_t)8192 * 16 * sizeof(double)))) return bail(st);
   if ((st = alloc((void**)&e->rb.counter, 64))) return bail(st);
   {
-    // a block of 256 threads per 4096 sites of a run, at most 32 a run
+    // a block of 256 threads per 4096 sites of a run, at most 64 a run
     std::vector<EnsEnergyRun> runs(nruns);
     int mb = 1;
     for (int r = 0; r < nruns; ++r) {
       const auto& c = e->cls[e->run_cls[r]];
       const int64_t n3 = (int64_t)c.n * c.n * c.n;
-      runs[r] = EnsEnergyRun{e->run_off[r], e->run_fk[r], c.dk * c.dk, c.n, (int)std::min<int64_t>(32, (n3 + 4095) / 4096)};
+      runs[r] = EnsEnergyRun{e->run_off[r], e->run_fk[r], c.dk * c.dk, c.n, (int)std::min<int64_t>(64, (n3 + 4095) / 4096)};
       mb = std::max(mb, runs[r].blocks);
     }
     const size_t nr = (size_t)nruns, tab = sizeof(EnsEnergyRun) * nr;

@@ -88,42 +88,55 @@ __global__ void __launch_bounds__(256) bin_kernel(BinArgs a) {
   for (int row = blockIdx.x * nw + warp; row < nrow; row += gridDim.x * nw) {
     const int jj = row % hy, kk = row / hy, r2 = jj * jj + kk * kk;
     const int my = (jj == 0 || 2 * jj == a.ny) ? 1 : 2, mz = (kk == 0 || 2 * kk == a.nz) ? 1 : 2;
+    size_t at[4];  // the rows (+-y, +-z)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int y = my == 2 && (r & 1) ? a.ny - jj : jj, z = (my == 2 ? r >> 1 : r) ? a.nz - kk : kk;
+      at[r] = ((size_t)z * a.ny + y) * hx;
+    }
     for (int x0 = 0; x0 < hx; x0 += 32) {
       const int x = x0 + lane;
       const bool on = x < hx;
       const int m2 = r2 + x * x, l = on ? isqrt_exact(m2) : 0x40000000 + lane;
       double v = 0.0, vi = 0.0;
-      if (on) {
-        for (int iz = 0; iz < mz; ++iz) {
-#pragma unroll 2
-          for (int iy = 0; iy < my; ++iy) {
-            const int y = iy ? a.ny - jj : jj, z = iz ? a.nz - kk : kk;
-            const size_t m = ((size_t)z * a.ny + y) * hx + x;
-            if constexpr (KIND == BIN_GW) {
-              if (l < nb) {
-                C h[6];
+      if constexpr (KIND == BIN_GW) {
+        if (on && l < nb) {
+          for (int r = 0; r < my * mz; ++r) {
+            C h[6];
 #pragma unroll
-                for (int i = 0; i < 6; ++i) h[i] = static_cast<const C*>(a.F[i])[m];
-                v += tt_power(h, __ldg(a.sins + x), __ldg(a.sins + hx + y), __ldg(a.sins + hx + a.ny + z));
-              }
-            } else {
-              const C f = F1[m];
-              const double fr = widen(f.x), fi = widen(f.y);
-              if constexpr (KIND == BIN_CROSS) {
-                const C g = F2[m];
-                const double gr = widen(g.x), gi = widen(g.y);
-                v = fma(fi, gi, fma(fr, gr, v));     // Re(F1 conj F2)
-                vi = fma(-fr, gi, fma(fi, gr, vi));  // Im(F1 conj F2)
-              } else {
-                v = fma(fi, fi, fma(fr, fr, v));
-              }
-            }
+            for (int i = 0; i < 6; ++i) h[i] = static_cast<const C*>(a.F[i])[at[r] + x];
+            const int y = (r & 1) && my == 2 ? a.ny - jj : jj, z = r >= my ? a.nz - kk : kk;
+            v += tt_power(h, __ldg(a.sins + x), __ldg(a.sins + hx + y), __ldg(a.sins + hx + a.ny + z));
           }
         }
-        if (x != 0 && 2 * x != a.nx) {
-          v += v;
-          vi += vi;
+      } else {
+        // the mirrored rows' values in flight together
+        C f[4], g[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          f[r] = C{0, 0};
+          g[r] = C{0, 0};
+          if (on && r < my * mz) {
+            f[r] = F1[at[r] + x];
+            if constexpr (KIND == BIN_CROSS) g[r] = F2[at[r] + x];
+          }
         }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          if (r >= my * mz) break;
+          const double fr = widen(f[r].x), fi = widen(f[r].y);
+          if constexpr (KIND == BIN_CROSS) {
+            const double gr = widen(g[r].x), gi = widen(g[r].y);
+            v = fma(fi, gi, fma(fr, gr, v));     // Re(F1 conj F2)
+            vi = fma(-fr, gi, fma(fi, gr, vi));  // Im(F1 conj F2)
+          } else {
+            v = fma(fi, fi, fma(fr, fr, v));
+          }
+        }
+      }
+      if (x != 0 && 2 * x != a.nx) {
+        v += v;
+        vi += vi;
       }
       double s[NS];
       if constexpr (KIND == BIN_POWER || KIND == BIN_CROSS) {

@@ -26,14 +26,13 @@ template <typename R, int NF, typename Acc>
 __device__ __forceinline__ void site_sums(const R* phi, const R* pi, int64_t fs, int64_t t, int64_t tend, int64_t step,
                                           const ModelP& m, Acc (&s)[4]) {
   for (; t < tend; t += step) {
-    R f[NF], ke = R(0);
+    R f[NF];
 #pragma unroll
     for (int l = 0; l < NF; ++l) {
       f[l] = phi[l * fs + t];
       const R p = pi[l * fs + t];
-      ke += p * p;
+      s[0].add(p * p);
     }
-    s[0].add(ke);
     s[1].add(model_v<R, NF>(m, f));
     s[2].add(f[0]);
     if (NF > 1) s[3].add(f[NF - 1]);
@@ -105,15 +104,16 @@ __global__ void __launch_bounds__(256) energy_kernel(EnergyArgs a) {
 }
 
 // ------------------------------------------------------------- stencils
-// Finite-difference lattices: red[0..3], red[4] = -sum phi L phi, red[5] = sum
+// FP64 finite-difference lattices: red[0..3], red[4] = -sum phi L phi, red[5] = sum
 // of the squared differences and, with strains, red[6] = sum w pu^2, red[7] =
 // -sum w u L u (w = 2 off the diagonal), over planes [zlo, zhi).  A thread
 // marches along z with the centre and the face- and corner-neighbour sums of
 // three planes in registers, so a plane is read once (9 values instead of 27
 // per site); each pair of neighbours enters the squared differences once, at
 // its lower site, for both.
-template <typename R, int NF, bool GW, bool SEVEN>
+template <int NF, bool GW, bool SEVEN>
 __global__ void __launch_bounds__(128) fd_energy_kernel(EnergyArgs a, int zlo, int zhi, int zc) {
+  using R = double;
   constexpr int NC = NF + (GW ? 6 : 0);
   using Acc = typename AccOf<R>::type;
   Acc s[8];
@@ -227,6 +227,101 @@ __global__ void __launch_bounds__(128) fd_energy_kernel(EnergyArgs a, int zlo, i
   }
 }
 
+// The same sums of FP32 lattices.  An FP32 term's rounding is part of the
+// result (1e-9 of an energy), so every site's neighbours are added in the order
+// of the reference's loops; a thread keeps three planes of one array's 3 x 3
+// values (9 reads a site instead of 27) and takes the arrays one after another.
+template <int NF, bool GW, bool SEVEN>
+__global__ void __launch_bounds__(128) fd_energy32_kernel(EnergyArgs a, int zlo, int zhi, int zc) {
+  using R = float;
+  constexpr int NC = NF + (GW ? 6 : 0);
+  KSum s[8];
+  const int nx = a.nx, ny = a.ny, nz = a.nz;
+  const int64_t N = (int64_t)nx * ny * nz, plane = (int64_t)nx * ny;
+  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 4 + threadIdx.y;
+  const int z0 = zlo + blockIdx.z * zc, z1 = min(z0 + zc, zhi);
+  if (x < nx && y < ny) {
+    const int col[3] = {x ? x - 1 : nx - 1, x, x + 1 < nx ? x + 1 : 0};
+    const int row[3] = {(y ? y - 1 : ny - 1) * nx, y * nx, (y + 1 < ny ? y + 1 : 0) * nx};
+    const R c0 = (R)a.c[0], c1 = (R)a.c[1], c2 = (R)a.c[2], c3 = (R)a.c[3];
+    auto wrap = [&](int z) { return z < 0 ? z + nz : (z >= nz ? z - nz : z); };
+#pragma unroll 1
+    for (int c = 0; c < NC; ++c) {
+      const R* g = c < NF ? static_cast<const R*>(a.phi) + c * N : static_cast<const R*>(a.u) + (c - NF) * N;
+      R v[3][3][3];
+      auto load = [&](int z, R (&w)[3][3]) {
+        const R* gz = g + (int64_t)wrap(z) * plane;
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+            if (!SEVEN || i == 1 || j == 1) w[j][i] = __ldg(gz + row[j] + col[i]);
+      };
+      load(z0 - 1, v[0]);
+      load(z0, v[1]);
+      for (int z = z0; z < z1; ++z) {
+        load(z + 1, v[2]);
+        const int64_t t = (int64_t)z * plane + row[1] + x;
+        const R g0 = v[1][1][1];
+        R r1 = 0, r2 = 0, r3 = 0, q1 = 0, q2 = 0, q3 = 0;
+#pragma unroll
+        for (int dz = 0; dz < 3; ++dz)
+#pragma unroll
+          for (int dy = 0; dy < 3; ++dy)
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx) {
+              const int rank = (dx != 1) + (dy != 1) + (dz != 1);
+              if (rank == 0 || (SEVEN && rank > 1)) continue;
+              const R w = v[dz][dy][dx], d = w - g0;
+              if (rank == 1) { r1 += w; q1 += d * d; }
+              else if (rank == 2) { r2 += w; q2 += d * d; }
+              else { r3 += w; q3 += d * d; }
+            }
+        const R lapsum = c0 * g0 + c1 * r1 + c2 * r2 + c3 * r3;
+        if (c < NF) {
+          const R grad2 = c1 * q1 + c2 * q2 + c3 * q3;
+          const R p = static_cast<const R*>(a.pi)[c * N + t];
+          s[0].add(p * p);
+          s[4].add(-g0 * lapsum);
+          s[5].add(grad2);
+          if (c == 0) {
+            R f[NF];
+            f[0] = g0;
+            if (NF > 1) f[NF - 1] = static_cast<const R*>(a.phi)[(NF - 1) * N + t];
+            s[1].add(model_v<R, NF>(a.model, f));
+            s[2].add(f[0]);
+            if (NF > 1) s[3].add(f[NF - 1]);
+          }
+        } else {
+          const R w = c - NF < 3 ? R(1) : R(2);
+          const R p = static_cast<const R*>(a.pu)[(c - NF) * N + t];
+          s[6].add(w * p * p);
+          s[7].add(-w * g0 * lapsum);
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            v[0][j][i] = v[1][j][i];
+            v[1][j][i] = v[2][j][i];
+          }
+      }
+    }
+  }
+  constexpr int NV = GW ? 8 : 6;
+  FF v[NV];
+  double tot[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) v[i] = s[i].red();
+  if (grid_reduce<NV>(v, a.rb, tot)) {
+    for (int i = 0; i < NV; ++i) {
+      a.sc->red[i] = tot[i];
+      if (bad(tot[i])) a.sc->err |= 1u;
+    }
+    for (int i = NV; i < 8; ++i) a.sc->red[i] = 0.0;
+  }
+}
+
 // LOG.out's ball: over the sites with |(x, y, z) + 1 - n/2|^2 dx^2 < ball_r2
 // (1-based indices about n/2, iofile.f90:552) red[9] = sum (sum_f pi_f)^2,
 // red[10] = the stencil's gradient squared, red[11] = V
@@ -292,13 +387,19 @@ int energy_go(const EnergyArgs& a, cudaStream_t s) {
   const int want = std::max(1, (8 * (a.grid / 4) + gx * gy - 1) / (gx * gy));
   const int zc = std::max(2, (zhi - zlo + want - 1) / want);
   const dim3 grid(gx, gy, (zhi - zlo + zc - 1) / zc), block(32, 4);
+#define LAT_FD_ENERGY(GWV, SEV)                                                                          \
+  do {                                                                                                  \
+    if constexpr (sizeof(R) == 8) fd_energy_kernel<NF, GWV, SEV><<<grid, block, 0, s>>>(a, zlo, zhi, zc); \
+    else fd_energy32_kernel<NF, GWV, SEV><<<grid, block, 0, s>>>(a, zlo, zhi, zc);                        \
+  } while (0)
   if (a.u) {
-    if (seven) fd_energy_kernel<R, NF, true, true><<<grid, block, 0, s>>>(a, zlo, zhi, zc);
-    else fd_energy_kernel<R, NF, true, false><<<grid, block, 0, s>>>(a, zlo, zhi, zc);
+    if (seven) LAT_FD_ENERGY(true, true);
+    else LAT_FD_ENERGY(true, false);
   } else {
-    if (seven) fd_energy_kernel<R, NF, false, true><<<grid, block, 0, s>>>(a, zlo, zhi, zc);
-    else fd_energy_kernel<R, NF, false, false><<<grid, block, 0, s>>>(a, zlo, zhi, zc);
+    if (seven) LAT_FD_ENERGY(false, true);
+    else LAT_FD_ENERGY(false, false);
   }
+#undef LAT_FD_ENERGY
   const int st = done("energy");
   if (st != LAT_OK || !(a.ball_r2 > 0.0)) return st;
   ball_kernel<R, NF><<<a.grid, 256, 0, s>>>(a);
@@ -318,14 +419,24 @@ __device__ __forceinline__ void parseval_rows(const C* F, int nx, int ny, int nz
     const int jj = row % hy, kk = row / hy;
     const R kyz = (R)((double)(jj * jj) * dky2 + (double)(kk * kk) * dkz2);
     const int my = (jj == 0 || 2 * jj == ny) ? 1 : 2, mz = (kk == 0 || 2 * kk == nz) ? 1 : 2;
+    size_t at[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int y = my == 2 && (r & 1) ? ny - jj : jj, z = (my == 2 ? r >> 1 : r) ? nz - kk : kk;
+      at[r] = ((size_t)z * ny + y) * hx;
+    }
+#pragma unroll 2
     for (int x = lane; x < hx; x += 32) {
+      C v[4];  // in flight together
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        v[r] = C{0, 0};
+        if (r < my * mz) v[r] = F[at[r] + x];
+      }
       R t = R(0);
-      for (int iz = 0; iz < mz; ++iz)
-        for (int iy = 0; iy < my; ++iy) {
-          const int y = iy ? ny - jj : jj, z = iz ? nz - kk : kk;
-          const C v = F[((size_t)z * ny + y) * hx + x];
-          t += v.x * v.x + v.y * v.y;
-        }
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (r < my * mz) t += v[r].x * v[r].x + v[r].y * v[r].y;
       if (x != 0 && 2 * x != nx) t += t;
       acc.add(((R)(x * x) * dkx2 + kyz) * t);
     }
