@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(256) pw_kernel(PwArgs a) {
     }
   };
 
-  const int64_t nvec = N / 4;
+  // four sites per access where the second field's array is 16-byte aligned too
+  const int64_t nvec = (NF == 1 || N % (16 / (int)sizeof(R)) == 0) ? N / 4 : 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += stride) {
     const int64_t s0 = v * 4;
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(256) pw_kernel(PwArgs a) {
       if (MODE != PW_DRIFT) P[l].store(pi + l * N + s0);
     }
   }
-  // tail (N not a multiple of 4)
+  // tail (N not a multiple of 4), or all sites one by one
   for (int64_t s = nvec * 4 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < N; s += stride) {
     R f[NF], c[NF], p[NF], lp[NF], dl[NF];
 #pragma unroll
