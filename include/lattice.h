@@ -102,9 +102,9 @@ typedef struct lat_config {
  * and C2R (any size).  SEPARABLE: three passes of in-register 1D transforms,
  * one per axis (sides 16..512, powers of two), which also transform the FP32
  * field with its Kahan compensation.  AUTO: until lat_autotune times both on
- * the handle's lattice and keeps the faster, FP64 lattices with power-of-two
- * sides 16..512 run the passes (two fields: any such sides; one field: nx >=
- * 64), all others cuFFT. */
+ * the handle's lattice and keeps the faster, FP64 lattices whose sides are 9..256
+ * or powers of two up to 512 run the passes (one field: more than 32^3 sites),
+ * all others cuFFT. */
 enum lat_spectral_impl { LAT_SPEC_IMPL_AUTO = 0, LAT_SPEC_IMPL_CUFFT = 1, LAT_SPEC_IMPL_SEPARABLE = 2 };
 
 typedef struct lat_s lat_t;

@@ -24,7 +24,7 @@
 
 #include "bin.hpp"
 #include "engine.hpp"
-#include "fx.cuh"
+#include "fx_host.hpp"
 #include "integrator.hpp"
 #include "net.hpp"
 
@@ -130,8 +130,11 @@ struct lat_s {
   bool fx_ok = false;             // FP64: the fixed-point passes (k_fx.cuh) tile these sizes
   bool sep_stream = true;         // streamed passes where available (LAT_SEP_CLASSIC=1: off)
   void* tw[3] = {nullptr, nullptr, nullptr};  // W_N^j per axis, FP32 (k_sep.cuh)
-  fx::Tw* fxtw[3] = {nullptr, nullptr, nullptr};  // and as split integers (one allocation): sides the fixed-point
-                                                  // transforms take, else null
+  fx::Tw* fxmem = nullptr;                        // tables of the fixed-point transforms
+  fx::Tw* fxtw[3] = {nullptr, nullptr, nullptr};  // W_N^j as split integers, power-of-two sides
+  fx::Tw* fxpad[3] = {nullptr, nullptr, nullptr}; // FP64 lattices' other sides: W_M^j and the multiplier of M points
+  int fxm[3] = {0, 0, 0};                         // M of such a side
+  bool fxr_ok = false;                            // the real-to-complex transform takes these sides
 
   int fd_ty = 8, fd_zc = 32;
   int pw_grid = 0, pw_block = 256;
@@ -240,13 +243,16 @@ int n_terms(const lat_s* h) {
 bool fx_side(int n) { return n >= 16 && n <= 512 && (n & (n - 1)) == 0; }
 
 // Whether an AUTO lattice takes the separable passes before any autotuning:
-// FP64 lattices that the fixed-point passes tile.  A Yoshida-4 step of two
-// expanding fields: 0.11 ms against 0.24 ms on cuFFT at 32^3, 4.7 against 24.8
-// at 256^3.  One-field lattices with rows of one tile (32 sites) keep cuFFT,
-// which AUTO has always reported for them; so do FP32 lattices, whose passes
-// round their fields differently (lat_autotune or SEPARABLE choose them).
+// FP64 lattices that the fixed-point passes take, direct (a Yoshida-4 step of
+// two expanding fields: 0.11 ms against 0.24 ms on cuFFT at 32^3, 4.7 against
+// 24.8 at 256^3) or padded (a kick of two expanding fields: 33 us against 64 at
+// 24^3, 370 against 929 at 150 x 108 x 96, 2.2 ms against 3.8 at 192^3, the
+// least favourable side, 472 us against 4096 at 127 x 131 x 113).  One-field
+// lattices of up to 32^3 sites keep cuFFT, which AUTO has always reported for
+// them; so do FP32 lattices, whose passes round their fields differently
+// (lat_autotune or SEPARABLE choose them).
 bool auto_separable(const lat_s* h) {
-  return h->fx_ok && (h->nf == 2 || h->nx >= 64) && !getenv_flag("LAT_NO_SEPARABLE");
+  return h->fx_ok && (h->nf == 2 || h->N > 32768) && !getenv_flag("LAT_NO_SEPARABLE");
 }
 
 // Tile of the stencil passes before any autotuning: 4 rows, and the chunk of
@@ -291,6 +297,58 @@ int fft_exec_c2r(lat_s* h, cufftHandle p, void* in, void* out) {
   Timed t(h, LAT_K_FFT_C2R);
   if (h->prec == LAT_FP64) CF(cufftExecZ2D(p, (cufftDoubleComplex*)in, (cufftDoubleReal*)out));
   else CF(cufftExecC2R(p, (cufftComplex*)in, (cufftReal*)out));
+  return LAT_OK;
+}
+
+// Tables and availability of the fixed-point transforms: the spectral passes
+// of FP64 lattices, whose power-of-two sides run directly where their lines
+// fill whole tiles of 16 (pairs of lines with one field) and whose other sides
+// up to 256 run padded, and the real-to-complex transform of power-of-two
+// lattices.
+int make_fx_tables(lat_s* h) {
+  const int dims[3] = {h->nx, h->ny, h->nz};
+  const int tile = h->nf == 2 ? 16 : 32;
+  h->fxr_ok = fx_side(h->nx) && fx_side(h->ny) && fx_side(h->nz);
+  const bool passes = h->prec == LAT_FP64 && spectral(h);
+  h->fx_ok = passes;
+  size_t at[3] = {0, 0, 0}, pad[3] = {0, 0, 0}, tot = 0;
+  for (int ax = 0; ax < 3; ++ax) {
+    const int n = dims[ax];
+    const int64_t lines = h->N / n;
+    if (fx_side(n)) {
+      at[ax] = tot;
+      tot += n;
+    }
+    if (!passes || (fx_side(n) && lines % tile == 0 && (ax == 0 || h->nx % tile == 0))) continue;
+    if (n < 9 || n > 256) {
+      h->fx_ok = false;
+      continue;
+    }
+    int m = 64;
+    while (m < 2 * n - 1) m *= 2;
+    h->fxm[ax] = m;
+    pad[ax] = tot;
+    tot += m + m / 4 + 1;
+  }
+  if (!h->fx_ok) {
+    for (int ax = 0; ax < 3; ++ax) h->fxm[ax] = 0;
+    if (!h->fxr_ok) return LAT_OK;
+  }
+  std::vector<fx::Tw> w(tot);
+  for (int ax = 0; ax < 3; ++ax) {
+    if (fx_side(dims[ax])) fx::roots(dims[ax], &w[at[ax]]);
+    if (h->fxm[ax]) {
+      fx::roots(h->fxm[ax], &w[pad[ax]]);
+      fx::multiplier(dims[ax], h->fxm[ax], &w[pad[ax]], reinterpret_cast<fx::Mult*>(&w[pad[ax] + h->fxm[ax]]));
+    }
+  }
+  if (cudaMalloc(&h->fxmem, tot * sizeof(fx::Tw)) != cudaSuccess) return set_error(LAT_ERR_ALLOC, "transform tables");
+  CK(cudaMemcpyAsync(h->fxmem, w.data(), tot * sizeof(fx::Tw), cudaMemcpyHostToDevice, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  for (int ax = 0; ax < 3; ++ax) {
+    if (fx_side(dims[ax])) h->fxtw[ax] = h->fxmem + at[ax];
+    if (h->fxm[ax]) h->fxpad[ax] = h->fxmem + pad[ax];
+  }
   return LAT_OK;
 }
 
@@ -662,7 +720,7 @@ int sep_pass(lat_s* h, int axis, double hk, double hg, double hd, int* grid_out 
     a.lap = axis == 2 ? h->lap_alt : h->lap;
     a.lap_out = axis == 0 ? h->lap : h->lap_alt;
   }
-  a.twN = fx ? static_cast<const void*>(h->fxtw[axis]) : h->tw[axis];
+  a.twN = !fx ? h->tw[axis] : static_cast<const void*>(h->fxm[axis] ? h->fxpad[axis] : h->fxtw[axis]);
   if (!(fx ? h->fx_ok : h->sep_ok) || !a.twN || !a.phi || !a.phi_out || !a.pi || !a.pi_out || !a.lap || !a.lap_out ||
       (h->prec == LAT_FP32_KAHAN && (!a.phic || !a.phic_out)))
     return set_error(LAT_ERR_STATE, "separable pass buffers missing");
@@ -698,6 +756,16 @@ int sep_pass(lat_s* h, int axis, double hk, double hg, double hd, int* grid_out 
   // a non-finite field is reported by the expanding lattices' Friedmann sums
   // and on lattices that asked for the separable passes
   a.nan_flag = a.conf || h->cfg.spectral_impl == LAT_SPEC_IMPL_SEPARABLE;
+  if (fx && h->fxm[axis]) {
+    const int64_t real = h->N / n;
+    a.nlines = h->nf == 2 ? real : (real + 1) / 2;
+    switch (h->fxm[axis]) {
+      case 64: return launch_fxg_64(a, axis, h->stream);
+      case 128: return launch_fxg_128(a, axis, h->stream);
+      case 256: return launch_fxg_256(a, axis, h->stream);
+      default: return launch_fxg_512(a, axis, h->stream);
+    }
+  }
   if (fx) {
     switch (n) {
       case 16: return launch_fx_16(a, axis, h->stream);
@@ -1013,7 +1081,7 @@ int compute_energies(lat_s* h, double* out, double ball_r2 = 0.0, double* ball =
     RET(launch_energy(e, h->prec, h->stream));
   }
   if (spectral(h)) {
-    if (h->prec == LAT_FP64 && h->fxtw[0]) {
+    if (h->prec == LAT_FP64 && h->fxr_ok) {
       for (int l = 0; l < h->nf; ++l)
         RET(fx_r2c(h, (const double*)h->fld[h->cur] + l * h->N, nullptr, (double2*)h->Fk + l * h->M));
     } else {
@@ -1082,14 +1150,14 @@ int output_spectrum(lat_s* h, int what, int field, int slot, void** Fout, int* p
   RET(src_ptr(h, what, field, &src));
   if (h->prec == LAT_FP64) {
     void* F = (char*)h->Fk + (size_t)slot * h->M * h->csz;
-    if (h->fxtw[0]) RET(fx_r2c(h, src, nullptr, static_cast<double2*>(F)));
+    if (h->fxr_ok) RET(fx_r2c(h, src, nullptr, static_cast<double2*>(F)));
     else RET(fft_exec_r2c(h, h->p_r2c1, src, F));
     *Fout = F;
     *prec = LAT_FP64;
     return LAT_OK;
   }
   if (!h->Fk64) CK(cudaMalloc(&h->Fk64, (size_t)2 * h->M * sizeof(double2)));
-  if (h->fxtw[0]) {
+  if (h->fxr_ok) {
     const void* cmp = (what == LAT_SPEC_FLD && h->fldc) ? (const char*)h->fldc + (size_t)field * h->N * h->rsz : nullptr;
     double2* F = static_cast<double2*>(h->Fk64) + (size_t)slot * h->M;
     RET(fx_r2c(h, src, cmp, F));
@@ -1235,7 +1303,7 @@ int lat_destroy(lat_t* h) {
   if (h->cl_stream) cudaStreamDestroy(h->cl_stream);
   for (void* t : h->tw)
     if (t) cudaFree(t);
-  if (h->fxtw[0]) cudaFree(h->fxtw[0]);
+  if (h->fxmem) cudaFree(h->fxmem);
   h->bins.free();
   {
     void* cb[] = {h->cl_b.a0, h->cl_b.a1, h->cl_b.a2, h->cl_b.out};
@@ -1373,9 +1441,6 @@ int lat_create(lat_t** out, const lat_config* cfg) {
     if (h->sep_ok) h->sep_ok = h->nx % cols(h->ny) == 0 && h->nx % cols(h->nz) == 0;
     if (cfg->spectral_impl == LAT_SPEC_IMPL_SEPARABLE && !h->sep_ok)
       return bail(set_error(LAT_ERR_UNSUPPORTED, "separable spectral passes need power-of-two sides 16..512"));
-    // FP64: 16 complex lines per tile (x-columns: 16 with two fields, 32 with one)
-    h->fx_ok = h->prec == LAT_FP64 && fx_side(h->nx) && fx_side(h->ny) && fx_side(h->nz) &&
-               h->nx % (h->nf == 2 ? 16 : 32) == 0;
     h->sep = h->sep_ok && cfg->spectral_impl == LAT_SPEC_IMPL_SEPARABLE && !getenv_flag("LAT_NO_SEPARABLE");
     // two FP32 fields on lines of 128 or 256 points whose passes all form
     // whole tiles: the streamed passes (LAT_SEP_CLASSIC=1 keeps the others)
@@ -1386,7 +1451,6 @@ int lat_create(lat_t** out, const lat_config* cfg) {
     h->sep_stream = h->sep_ok && h->prec == LAT_FP32_KAHAN && h->nf == 2 && lx && ly && lz &&
                     ((int64_t)h->ny * h->nz) % lx == 0 && h->nx % ly == 0 && h->nx % lz == 0 &&
                     !getenv_flag("LAT_SEP_CLASSIC");
-    if (cfg->spectral_impl == LAT_SPEC_IMPL_AUTO) h->sep = auto_separable(h);
     if (h->sep_ok && h->prec != LAT_FP64) {
       if ((st = alloc(&h->fld[1], fb))) return bail(st);
       if (h->prec == LAT_FP32_KAHAN && (st = alloc(&h->fldc_alt, fb))) return bail(st);
@@ -1411,26 +1475,8 @@ int lat_create(lat_t** out, const lat_config* cfg) {
       }
     }
   }
-  if (fx_side(h->nx) && fx_side(h->ny) && fx_side(h->nz)) {
-    const int dims[3] = {h->nx, h->ny, h->nz};
-    std::vector<fx::Tw> w((size_t)h->nx + h->ny + h->nz);
-    if ((st = alloc((void**)&h->fxtw[0], w.size() * sizeof(fx::Tw)))) return bail(st);
-    size_t at = 0;
-    for (int ax = 0; ax < 3; ++ax) {
-      h->fxtw[ax] = h->fxtw[0] + at;
-      for (int j = 0; j < dims[ax]; ++j) {
-        const long double ang = -6.283185307179586476925286766559L * (long double)j / (long double)dims[ax];
-        const long double one = 4611686018427387904.0L;  // 2^62
-        const long long c = llrintl(cosl(ang) * one), sn = llrintl(sinl(ang) * one);
-        w[at + j] = fx::Tw{fx::split_hi(c), fx::split_lo(c), fx::split_hi(sn), fx::split_lo(sn)};
-      }
-      at += dims[ax];
-    }
-    if ((e = cudaMemcpyAsync(h->fxtw[0], w.data(), w.size() * sizeof(fx::Tw), cudaMemcpyHostToDevice, h->stream)) !=
-            cudaSuccess ||
-        (e = cudaStreamSynchronize(h->stream)) != cudaSuccess)
-      return bail(cuda_fail(e, "twiddle upload"));
-  }
+  if ((st = make_fx_tables(h))) return bail(st);
+  if (spectral(h) && cfg->spectral_impl == LAT_SPEC_IMPL_AUTO) h->sep = auto_separable(h);
   h->ev_pool.resize(4096);
   for (auto& ev : h->ev_pool) {
     cudaEventCreate(&ev.a);
@@ -1702,7 +1748,7 @@ int lat_gw_spectrum(lat_t* h, int32_t nbins, double* S, double* W) {
   if (nbins < 1 || nbins > kMaxBins) return set_error(LAT_ERR_ARG, "nbins out of range");
   ApiGuard g(h);
   if (!h->Fk6) CK(cudaMalloc(&h->Fk6, (size_t)6 * h->M * h->csz));
-  if (h->prec == LAT_FP64 && h->fxtw[0]) {
+  if (h->prec == LAT_FP64 && h->fxr_ok) {
     for (int k = 0; k < 6; ++k)
       RET(fx_r2c(h, (const double*)h->pu + k * h->N, nullptr, (double2*)h->Fk6 + k * h->M));
   } else {

@@ -152,6 +152,11 @@ int launch_fx_64(const SepArgs& a, int axis, cudaStream_t s);
 int launch_fx_128(const SepArgs& a, int axis, cudaStream_t s);
 int launch_fx_256(const SepArgs& a, int axis, cudaStream_t s);
 int launch_fx_512(const SepArgs& a, int axis, cudaStream_t s);
+// and for other sides, lines padded to 64 ... 512 points (k_fxg.cuh)
+int launch_fxg_64(const SepArgs& a, int axis, cudaStream_t s);
+int launch_fxg_128(const SepArgs& a, int axis, cudaStream_t s);
+int launch_fxg_256(const SepArgs& a, int axis, cudaStream_t s);
+int launch_fxg_512(const SepArgs& a, int axis, cudaStream_t s);
 // 3D real-to-complex transform in fixed point (k_fxr.cuh): rows, then lines along y and z
 int launch_fxr_rows_16(const void* hi, const void* c, int precision, void* F, int64_t nlines, const void* tw, int nsm,
                        cudaStream_t s);

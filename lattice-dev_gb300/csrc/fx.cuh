@@ -410,6 +410,40 @@ LAT_HD void phase2(int t, Cx64* sl, const Tw* t2, int drop) {
     });
   });
 }
+// Lines padded with zeros (k_fxg.cuh): the multiplier is a table of numbers
+// below 1 (2^-62 units, split; even, entries 0..N/2) and `drop` bits are dropped.
+struct alignas(8) Mult {
+  int h, l;
+};
+template <int N>
+LAT_HD void phase2_tab(int t, Cx64* sl, const Tw* t2, const Mult* H, int drop) {
+  constexpr int P = Split<N>::P, Q = Split<N>::Q, S = P + 1, G = Q / P;
+  // rounded: a floor's constant offset on all modes would meet at the first point
+  const i64 half = drop > 0 ? 1LL << (drop - 1) : 0;
+  static_for<G>([&](auto gg) {
+    const int kq = t + gg.value * P;
+    i64 ur[P], ui[P];
+    static_for<P>([&](auto tt) {
+      const Cx64 z = sl[kq * S + tt.value];
+      ur[tt.value] = z.x;
+      ui[tt.value] = z.y;
+    });
+    dft<P, false>(ur, ui);
+    static_for<P>([&](auto kp) {
+      const int k = kq + Q * kp.value;
+      const Mult h = H[2 * kp.value < P ? k : N - k];
+      ur[kp.value] = (rmul(ur[kp.value], h.h, h.l) + half) >> drop;
+      ui[kp.value] = (rmul(ui[kp.value], h.h, h.l) + half) >> drop;
+    });
+    dft<P, true>(ur, ui);
+    static_for<P>([&](auto mp) {
+      constexpr int m = mp.value;
+      if constexpr (m != 0) cmul<true>(ur[m], ui[m], t2[m * Q + kq]);
+      sl[kq * S + m] = Cx64{ur[m], ui[m]};
+    });
+  });
+}
+
 // Forward transform only: row kq of the scratch becomes Z[kq + Q kp], kp < P
 // (after phase 1 and a barrier; each row belongs to one thread).
 template <int N>

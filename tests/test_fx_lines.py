@@ -13,6 +13,7 @@ signed overflow anywhere ends the process.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import subprocess
 from pathlib import Path
 
@@ -21,6 +22,7 @@ import pytest
 
 HERE = Path(__file__).resolve().parent
 SIZES = [16, 32, 64, 128, 256, 512]
+PADDED = [9, 10, 17, 32, 33, 64, 65, 96, 128, 129, 150, 251, 256]  # run on 64 ... 512 points
 
 
 @pytest.fixture(scope="module")
@@ -30,14 +32,16 @@ def fx(tmp_path_factory):
                     "-fsanitize-undefined-trap-on-error", "-o", str(so), str(HERE / "fx_lines.cpp")], check=True)
     lib = C.CDLL(str(so))
     dp = C.POINTER(C.c_double)
-    lib.fx_line.argtypes = [C.c_int, dp, C.c_double, dp]
+    lib.fx_line.argtypes = [C.c_int, C.c_int, dp, C.c_double, dp]
     lib.fx_round.argtypes = [C.c_longlong]
     lib.fx_round.restype = C.c_double
 
-    def line(a, b, dk2=1.0):
+    def line(a, b, dk2=1.0, padded=False):
+        n = len(a)
+        m = max(64, 1 << (2 * n - 2).bit_length()) if padded else n
         x = np.ascontiguousarray(np.stack([a, b]), np.float64)
         out = np.empty_like(x)
-        assert lib.fx_line(x.shape[1], x.ctypes.data_as(dp), dk2, out.ctypes.data_as(dp)) == 0
+        assert lib.fx_line(n, m, x.ctypes.data_as(dp), dk2, out.ctypes.data_as(dp)) == 0
         return out
     line.round = lib.fx_round
     return line
@@ -94,14 +98,14 @@ def inputs(n, kind, rng):
 
 
 @pytest.mark.parametrize("kind", ["noise", "mean", "smooth", "spike", "nyquist", "aligned", "uneven", "tiny", "large"])
-@pytest.mark.parametrize("n", SIZES)
-def test_line_against_long_double(fx, n, kind):
+@pytest.mark.parametrize("n,padded", [(n, False) for n in SIZES] + [(n, True) for n in PADDED])
+def test_line_against_long_double(fx, n, padded, kind):
     rng = np.random.default_rng(n)
     c = kernel(n)
     worst = np.zeros(2)
     for _ in range(4):
         a, b = inputs(n, kind, rng)
-        out = fx(a, b)
+        out = fx(a, b, padded=padded)
         ref64 = fp64(a, b)
         for l, x in enumerate((a, b)):
             e = exact(x, c)
@@ -116,8 +120,9 @@ def test_line_against_long_double(fx, n, kind):
     assert worst[0] <= 1.1 * worst[1] + 8 * 2.0 ** -53
 
 
-@pytest.mark.parametrize("n", SIZES)
-def test_line_special_values(fx, n):
+@pytest.mark.parametrize("n,padded", [(n, False) for n in SIZES] + [(n, True) for n in PADDED])
+def test_line_special_values(fx, n, padded):
+    fx = functools.partial(fx, padded=padded)
     z = np.zeros(n)
     assert np.array_equal(fx(z, z), np.zeros((2, n)))
     c = np.full(n, -0.7)

@@ -21,6 +21,12 @@ CASES = [((16, 16, 16), 2), ((32, 512, 16), 2), ((16, 32, 512), 2), ((512, 16, 3
          ((64, 64, 64), 1), ((512, 64, 32), 1), ((128, 512, 16), 1), ((128, 16, 512), 1), ((256, 128, 64), 1)]
 
 
+# sides that run padded (k_fxg.cuh): both edges of every padded length (9..32 on 64 points,
+# 33..64, 65..128, 129..256), odd numbers of lines with one field, padded beside direct sides
+CASES += [((9, 32, 33), 2), ((64, 65, 20), 2), ((17, 129, 12), 2), ((256, 9, 30), 2), ((48, 36, 255), 2),
+          ((65, 39, 13), 1), ((128, 33, 15), 1), ((150, 96, 10), 1), ((64, 18, 128), 1)]
+
+
 def pair(engine, shape, nf, **kw):
     out = []
     for impl in (L.SPEC_IMPL_AUTO, L.SPEC_IMPL_CUFFT):
