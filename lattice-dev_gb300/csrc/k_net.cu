@@ -414,33 +414,48 @@ __global__ void __launch_bounds__(256) out_conv_kernel(ConvArgs a, int zc) {
 // part[blk][tap][i][o] = sum over the block's sites s of X[s + off(tap)][i] * D[s][o]
 // (X: CX channels, halo-shifted; D: CD channels).  The GEMM's M side is the
 // 32-channel operand.  part_b[blk][o] = sum_s D[s][o].
-template <int CX, int CD>
-__global__ void __launch_bounds__(288) wgrad_kernel(WgradArgs a) {
+//
+// A warp owns three taps (dz = 0, 1, 2 of one (dy, dx)) and WM of the two
+// m-tiles, so a D fragment serves three taps' products; two slots per block
+// hide the copies.  Bound by mma.sync itself where both sides have 32 channels
+// (one m16n8k16 per SM in 4 clocks): 9 warps of two m-tiles leave a scheduler
+// with three warps and three with two, 18 warps of one m-tile do not (245 ->
+// 222 us).  Four 64^3 lattices, before (copies in line, a fragment of D per
+// tap, one thread per channel for part_b) and now: 32x32 300 -> 222 us, 32x8
+// 213 -> 107, 8x32 167 -> 63.
+template <int CX, int CD, int WM>
+__global__ void __launch_bounds__(288 * 2 / WM) wgrad_kernel(WgradArgs a) {
   constexpr bool MX = CX == 32;  // M = X channels (else M = D channels)
   constexpr int CN = MX ? CD : CX;
   constexpr int NT = CN / 8;
   constexpr int SX = Row<CX>::S, SD = Row<CD>::S;
   extern __shared__ __align__(16) unsigned char smraw[];
-  __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smraw);  // [HSITES][SX]
-  __nv_bfloat16* ds = xs + HSITES * SX;                           // [TSITES][SD]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;  // 9 warps
+  // two slots of a tile's X halo [HSITES][SX] and D [TSITES][SD]: the next
+  // tile's copies run behind this one's products
+  __nv_bfloat16* const xbuf = reinterpret_cast<__nv_bfloat16*>(smraw);
+  __nv_bfloat16* const dbuf = xbuf + 2 * HSITES * SX;
+  const int tid = threadIdx.x, lane = tid & 31, warp = (tid >> 5) % 9;
+  const int m0 = WM * ((tid >> 5) / 9);  // the warp's first m-tile of 16 channels
   const int g = lane >> 2, t4 = lane & 3;
-  float acc[3][2][NT][4];
+  float acc[3][WM][NT][4];
 #pragma unroll
   for (int j = 0; j < 3; ++j)
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int mt = 0; mt < WM; ++mt)
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[j][mt][nt][q] = 0.f;
-  float bsum = 0.f;  // thread tid < CD: channel tid of D
+  // column sums of D: thread tid < 256 adds channel tid % CD over its share of
+  // the tile's sites (one thread a channel held its warp's products up)
+  constexpr int BPARTS = 256 / CD, BSITES = TSITES / BPARTS;
+  float bsum = 0.f;
 
   const int tiles_x = a.nx / TX, tiles_y = a.ny / TY;
   const int64_t tiles_per = (int64_t)tiles_x * tiles_y * a.nz;
   const int64_t ntiles = tiles_per * a.nlat;
   const int64_t Nsite = (int64_t)a.nx * a.ny * a.nz;
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  auto stage = [&](int64_t tile, int slot) {
     const int64_t lat_i = tile / tiles_per;
     int64_t r = tile % tiles_per;
     const int tx = (int)(r % tiles_x);
@@ -448,66 +463,76 @@ __global__ void __launch_bounds__(288) wgrad_kernel(WgradArgs a) {
     const int ty = (int)(r % tiles_y);
     const int z0 = (int)(r / tiles_y);
     const int x0 = tx * TX, y0 = ty * TY;
-    __syncthreads();
-    load_halo<CX>(xs, a.x + lat_i * Nsite * CX, a.nx, a.ny, a.nz, x0, y0, z0);
-    {
-      constexpr int CH = CD / 8;
-      const __nv_bfloat16* D = a.d + lat_i * Nsite * CD;
-      for (int i = tid; i < TSITES * CH; i += blockDim.x) {
-        const int s = i / CH, c = i % CH;
-        const int xx = s % TX, yy = s / TX;
-        cp16(ds + s * SD + c * 8, D + (((int64_t)z0 * a.ny + y0 + yy) * a.nx + x0 + xx) * CD + c * 8);
-      }
+    load_halo<CX>(xbuf + slot * HSITES * SX, a.x + lat_i * Nsite * CX, a.nx, a.ny, a.nz, x0, y0, z0);
+    constexpr int CH = CD / 8;
+    const __nv_bfloat16* D = a.d + lat_i * Nsite * CD;
+    __nv_bfloat16* dst = dbuf + slot * TSITES * SD;
+    for (int i = tid; i < TSITES * CH; i += blockDim.x) {
+      const int s = i / CH, c = i % CH;
+      const int xx = s % TX, yy = s / TX;
+      cp16(dst + s * SD + c * 8, D + (((int64_t)z0 * a.ny + y0 + yy) * a.nx + x0 + xx) * CD + c * 8);
     }
+  };
+  if ((int64_t)blockIdx.x < ntiles) stage(blockIdx.x, 0);
+  cp_commit();
+  int slot = 0;
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, slot ^= 1) {
+    if (tile + gridDim.x < ntiles) stage(tile + gridDim.x, slot ^ 1);
     cp_commit();
-    cp_wait_all();
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     __syncthreads();
-    if (tid < CD)
-      for (int s = 0; s < TSITES; ++s) bsum += __bfloat162float(ds[s * SD + tid]);
-
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int tap = warp + 9 * j;
-      const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-#pragma unroll 1
-      for (int ky = 0; ky < TY; ++ky) {  // 16 sites of tile row ky per k-step
-        // shifted X rows: halo site of tile site (xx, ky) moved by the tap
-        auto xrow = [&](int xx) { return ((dz * HY) + (ky + dy)) * HX + (xx + dx); };
-        auto drow = [&](int xx) { return ky * TX + xx; };
-        const int idx = lane >> 3, rr = lane & 7;
-        // M operand (2 m-tiles of 16 channels): ldmatrix.trans of [site][chan]
-        uint32_t am[2][4];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-          const int site = rr + 8 * (idx >> 1), ch = mt * 16 + 8 * (idx & 1);
-          if constexpr (MX) ldsm_x4_t(am[mt], xs + xrow(site) * SX + ch);
-          else ldsm_x4_t(am[mt], ds + drow(site) * SD + ch);
-        }
-        // N operand (NT n-tiles of 8 channels)
-        uint32_t bn[NT][2];
-        if constexpr (NT >= 2) {
-#pragma unroll
-          for (int np = 0; np < NT / 2; ++np) {
-            const int site = rr + 8 * (idx & 1), ch = np * 16 + 8 * (idx >> 1);
-            uint32_t q[4];
-            if constexpr (MX) ldsm_x4_t(q, ds + drow(site) * SD + ch);
-            else ldsm_x4_t(q, xs + xrow(site) * SX + ch);
-            bn[2 * np][0] = q[0]; bn[2 * np][1] = q[1];
-            bn[2 * np + 1][0] = q[2]; bn[2 * np + 1][1] = q[3];
-          }
-        } else {
-          const int site = rr + 8 * (idx & 1);
-          uint32_t q[2];
-          if constexpr (MX) ldsm_x2_t(q, ds + drow(site) * SD);
-          else ldsm_x2_t(q, xs + xrow(site) * SX);
-          bn[0][0] = q[0]; bn[0][1] = q[1];
-        }
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-          for (int nt = 0; nt < NT; ++nt) mma16816(acc[j][mt][nt], am[mt], bn[nt][0], bn[nt][1]);
-      }
+    const __nv_bfloat16* xs = xbuf + slot * HSITES * SX;
+    const __nv_bfloat16* ds = dbuf + slot * TSITES * SD;
+    if (tid < 256) {
+      const __nv_bfloat16* q = ds + (tid / CD) * BSITES * SD + tid % CD;
+#pragma unroll 4
+      for (int s = 0; s < BSITES; ++s) bsum += __bfloat162float(q[s * SD]);
     }
+
+    // warp w's taps are (dy, dx) = (w / 3, w % 3) at dz = 0, 1, 2: one D
+    // fragment and three X fragments per 16 sites, then all their products
+    const int dy = warp / 3, dx = warp % 3;
+    const int idx = lane >> 3, rr = lane & 7;
+    const int ms = rr + 8 * (idx >> 1), mc = 8 * (idx & 1);                   // M side: site, channel
+    const int ns = rr + 8 * (idx & 1), nc = NT >= 2 ? 8 * (idx >> 1) : 0;     // N side
+    auto mfrag = [&](uint32_t (&am)[WM][4], const __nv_bfloat16* q, int S) {   // [site][chan] -> WM m-tiles
+#pragma unroll
+      for (int mt = 0; mt < WM; ++mt) ldsm_x4_t(am[mt], q + ms * S + (m0 + mt) * 16 + mc);
+    };
+    auto nfrag = [&](uint32_t (&bn)[NT][2], const __nv_bfloat16* q, int S) {  // NT n-tiles
+      if constexpr (NT >= 2) {
+#pragma unroll
+        for (int np = 0; np < NT / 2; ++np) {
+          uint32_t r[4];
+          ldsm_x4_t(r, q + ns * S + np * 16 + nc);
+          bn[2 * np][0] = r[0]; bn[2 * np][1] = r[1];
+          bn[2 * np + 1][0] = r[2]; bn[2 * np + 1][1] = r[3];
+        }
+      } else {
+        ldsm_x2_t(bn[0], q + ns * S);
+      }
+    };
+#pragma unroll 2
+    for (int ky = 0; ky < TY; ++ky) {  // 16 sites of tile row ky per k-step
+      const __nv_bfloat16* xr = xs + ((ky + dy) * HX + dx) * SX;
+      const __nv_bfloat16* dr = ds + ky * TX * SD;
+      uint32_t am[MX ? 3 : 1][WM][4], bn[MX ? 1 : 3][NT][2];
+      if constexpr (MX) nfrag(bn[0], dr, SD);
+      else mfrag(am[0], dr, SD);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        if constexpr (MX) mfrag(am[j], xr + j * HY * HX * SX, SX);
+        else nfrag(bn[j], xr + j * HY * HX * SX, SX);
+      }
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int mt = 0; mt < WM; ++mt)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+            mma16816(acc[j][mt][nt], am[MX ? j : 0][mt], bn[MX ? 0 : j][nt][0], bn[MX ? 0 : j][nt][1]);
+    }
+    __syncthreads();  // the slot is read before the copies after the next replace it
   }
   // partials in [tap][x-chan][d-chan] order
   float* part = a.part + (int64_t)blockIdx.x * 27 * CX * CD;
@@ -515,26 +540,49 @@ __global__ void __launch_bounds__(288) wgrad_kernel(WgradArgs a) {
   for (int j = 0; j < 3; ++j) {
     const int tap = warp + 9 * j;
 #pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
+    for (int mt = 0; mt < WM; ++mt)
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const int m = mt * 16 + g + 8 * (q >> 1), n = nt * 8 + 2 * t4 + (q & 1);
+          const int m = (m0 + mt) * 16 + g + 8 * (q >> 1), n = nt * 8 + 2 * t4 + (q & 1);
           const int i = MX ? m : n, o = MX ? n : m;
           part[(tap * CX + i) * CD + o] = acc[j][mt][nt][q];
         }
   }
-  if (tid < CD) a.part_b[(int64_t)blockIdx.x * CD + tid] = bsum;
+  __shared__ float bred[256];
+  if (tid < 256) bred[tid] = bsum;
+  __syncthreads();
+  if (tid < CD) {
+    float b = 0.f;
+    for (int k = 0; k < BPARTS; ++k) b += bred[k * CD + tid];
+    a.part_b[(int64_t)blockIdx.x * CD + tid] = b;
+  }
 }
 
-// grad[e] = sum over blocks of part[blk][e], blocks in index order
-__global__ void reduce_parts_kernel(const float* __restrict__ part, int nblk, int64_t per, float* __restrict__ out) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < per; e += (int64_t)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int b = 0; b < nblk; ++b) s += part[(int64_t)b * per + e];
-    out[e] = s;
+// grad[e] = sum over blocks of part[blk][e]: the weights, then the biases.
+// 16 threads take an element's blocks in turns, so that a few blocks' worth of
+// elements (the narrow layers) still keeps the reads of 12-17 MB in flight.
+constexpr int RP_PARTS = 16;
+__global__ void reduce_parts_kernel(const float* __restrict__ part, const float* __restrict__ part_b, int nblk,
+                                    int per, int per_b, float* __restrict__ out, float* __restrict__ out_b) {
+  __shared__ float red[RP_PARTS][33];
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int e = blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (e < per + per_b) {
+    const bool w = e < per;
+    const float* p = w ? part + e : part_b + (e - per);
+    const int64_t step = w ? per : per_b;
+#pragma unroll 8
+    for (int b = row; b < nblk; b += RP_PARTS) s += __ldg(p + b * step);
   }
+  red[row][lane] = s;
+  __syncthreads();
+  if (row || e >= per + per_b) return;
+  for (int k = 1; k < RP_PARTS; ++k) s += red[k][lane];
+  if (e < per) out[e] = s;
+  else out_b[e - per] = s;
 }
 
 // ------------------------------------------------------------ pointwise
@@ -612,11 +660,10 @@ __global__ void loss_kernel(LossArgs a) {
 }
 
 __global__ void sum_kernel(const double* __restrict__ part, int n, double* __restrict__ out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < n; ++i) s += part[i];
-    *out = s;
-  }
+  double s = 0.0;
+  for (int i = threadIdx.x; i < n; i += 32) s += part[i];
+  s = warp_sum(s);
+  if (threadIdx.x == 0) *out = s;
 }
 
 // Adam step on the flat FP32 parameters (bias-corrected)
@@ -737,31 +784,34 @@ int conv(const ConvArgs& a, int ca, int cb, int epi, int nsm, cudaStream_t s) {
   return set_error(LAT_ERR_UNSUPPORTED, "conv shape");
 }
 
-int wgrad_blocks(int nsm) { return nsm; }
+// Blocks of a weight-gradient pass: what fits an SM, one for 32 x 32 channels
+// (registers), two for 32 x 8 (90 KB of shared memory each) and three for
+// 8 x 32, which waits on its fragments and barriers otherwise.
+int wgrad_blocks(int nsm, int cx, int cd) { return nsm * (cx == 8 ? 3 : (cd == 8 ? 2 : 1)); }
 
-int wgrad(const WgradArgs& a, int cx, int cd, int nblk, float* dW, float* db, cudaStream_t s) {
+int wgrad(const WgradArgs& a, int cx, int cd, int nsm, float* dW, float* db, cudaStream_t s) {
   if (a.nx % TX || a.ny % TY) return set_error(LAT_ERR_ARG, "closure lattice: nx % 16, ny % 8");
-  size_t smem = 0;
   cudaError_t e;
-  auto go = [&](auto kern, int CX, int CD) -> int {
-    smem = (size_t)(HSITES * (CX == 32 ? 40 : 8) + TSITES * (CD == 32 ? 40 : 8)) * 2;
+  const int64_t ntiles = (int64_t)(a.nx / TX) * (a.ny / TY) * a.nz * a.nlat;
+  const int nblk = (int)std::min<int64_t>(ntiles, wgrad_blocks(nsm, cx, cd));
+  auto go = [&](auto kern, int CX, int CD, int WM) -> int {
+    const size_t smem = (size_t)(HSITES * (CX == 32 ? 40 : 8) + TSITES * (CD == 32 ? 40 : 8)) * 2 * 2;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_fail(e, "wgrad smem attribute");
-    kern<<<nblk, 288, smem, s>>>(a);
+    kern<<<nblk, 288 * 2 / WM, smem, s>>>(a);
     if (g_launch_counter) ++*g_launch_counter;
     e = cudaGetLastError();
     return e == cudaSuccess ? LAT_OK : cuda_fail(e, "wgrad launch");
   };
   int st;
-  if (cx == 32 && cd == 8) st = go(wgrad_kernel<32, 8>, 32, 8);
-  else if (cx == 32 && cd == 32) st = go(wgrad_kernel<32, 32>, 32, 32);
-  else if (cx == 8 && cd == 32) st = go(wgrad_kernel<8, 32>, 8, 32);
+  if (cx == 32 && cd == 8) st = go(wgrad_kernel<32, 8, 2>, 32, 8, 2);
+  else if (cx == 32 && cd == 32) st = go(wgrad_kernel<32, 32, 1>, 32, 32, 1);
+  else if (cx == 8 && cd == 32) st = go(wgrad_kernel<8, 32, 2>, 8, 32, 2);
   else return set_error(LAT_ERR_UNSUPPORTED, "wgrad shape");
   if (st != LAT_OK) return st;
-  const int64_t per = 27LL * cx * cd;
-  reduce_parts_kernel<<<(unsigned)((per + 255) / 256), 256, 0, s>>>(a.part, nblk, per, dW);
-  reduce_parts_kernel<<<1, 256, 0, s>>>(a.part_b, nblk, cd, db);
-  if (g_launch_counter) *g_launch_counter += 2;
+  const int per = 27 * cx * cd;
+  reduce_parts_kernel<<<(per + cd + 31) / 32, 32 * RP_PARTS, 0, s>>>(a.part, a.part_b, nblk, per, cd, dW, db);
+  if (g_launch_counter) ++*g_launch_counter;
   e = cudaGetLastError();
   return e == cudaSuccess ? LAT_OK : cuda_fail(e, "wgrad reduce launch");
 }

@@ -178,14 +178,13 @@ int loss_and_grad(lat_net_s* n, const float* data, int64_t stride, int nidx, int
   la.dout = n->d3;
   la.part = n->lpart;
   NRET(lat::net::loss(la, 2 * n->nsm, n->lsum, s));
-  const int nblk = wgrad_blocks(n->nsm);
   WgradArgs w{};
   w.nx = nx; w.ny = ny; w.nz = nz; w.nlat = nidx;
   w.part = n->part;
   w.part_b = n->part_b;
   // layer 3: input a2, gradient d3
   w.x = n->a2; w.d = n->d3;
-  NRET(wgrad(w, C_HID, C_OUT, nblk, n->G + OFF_W3, n->G + OFF_B3, s));
+  NRET(wgrad(w, C_HID, C_OUT, n->nsm, n->G + OFF_W3, n->G + OFF_B3, s));
   ConvArgs c{};
   c.nx = nx; c.ny = ny; c.nz = nz; c.nlat = nidx;
   c.err = n->err;
@@ -193,12 +192,12 @@ int loss_and_grad(lat_net_s* n, const float* data, int64_t stride, int nidx, int
   NRET(conv(c, C_OUT, C_HID, EPI_BWD, n->nsm, s));
   // layer 2
   w.x = n->a1; w.d = n->d2;
-  NRET(wgrad(w, C_HID, C_HID, nblk, n->G + OFF_W2, n->G + OFF_B2, s));
+  NRET(wgrad(w, C_HID, C_HID, n->nsm, n->G + OFF_W2, n->G + OFF_B2, s));
   c.in = n->d2; c.w = n->wb2; c.zin = n->z1; c.out = n->d1;
   NRET(conv(c, C_HID, C_HID, EPI_BWD, n->nsm, s));
   // layer 1
   w.x = n->a0; w.d = n->d1;
-  NRET(wgrad(w, C_IN, C_HID, nblk, n->G + OFF_W1, n->G + OFF_B1, s));
+  NRET(wgrad(w, C_IN, C_HID, n->nsm, n->G + OFF_W1, n->G + OFF_B1, s));
   if (loss) {
     NCK(cudaMemcpyAsync(loss, n->lsum, sizeof(double), cudaMemcpyDeviceToHost, s));
   }
@@ -300,9 +299,15 @@ int lat_net_create(lat_net_t** out, int32_t device, uint64_t seed) {
   const int64_t bn[] = {W1_N, W2_N, W3_N, W2_N, W3_N};
   for (int i = 0; i < 5; ++i)
     if ((e = cudaMalloc(bl[i], (size_t)bn[i] * 2)) != cudaSuccess) return bail(cuda_fail(e, "bf16 weights"));
-  const int nblk = wgrad_blocks(n->nsm);
-  if ((e = cudaMalloc(&n->part, (size_t)nblk * 27 * C_HID * C_HID * sizeof(float))) != cudaSuccess ||
-      (e = cudaMalloc(&n->part_b, (size_t)nblk * C_HID * sizeof(float))) != cudaSuccess ||
+  size_t parts = 0, parts_b = 0;  // partial gradients of the largest pass
+  const int wg[3][2] = {{C_HID, C_OUT}, {C_HID, C_HID}, {C_IN, C_HID}};
+  for (const auto& c : wg) {
+    const size_t nblk = wgrad_blocks(n->nsm, c[0], c[1]);
+    parts = std::max(parts, nblk * 27 * c[0] * c[1]);
+    parts_b = std::max(parts_b, nblk * c[1]);
+  }
+  if ((e = cudaMalloc(&n->part, parts * sizeof(float))) != cudaSuccess ||
+      (e = cudaMalloc(&n->part_b, parts_b * sizeof(float))) != cudaSuccess ||
       (e = cudaMalloc(&n->lpart, (size_t)2 * n->nsm * sizeof(double))) != cudaSuccess ||
       (e = cudaMalloc(&n->lsum, sizeof(double))) != cudaSuccess ||
       (e = cudaMalloc(&n->err, sizeof(int))) != cudaSuccess)

@@ -93,8 +93,8 @@ int conv(const ConvArgs& a, int ca, int cb, int epi, int nsm, cudaStream_t s);
 // backward data) and the 8-channel (4 padded) input layer; nx % 64 == 0 (rows of 128 or 64 sites)
 bool conv_tc_ok(int ca, int cb, int epi, int nx, int ny);
 int conv_tc(const ConvArgs& a, int ca, int epi, int nsm, int* err, cudaStream_t s);
-int wgrad_blocks(int nsm);
-int wgrad(const WgradArgs& a, int cx, int cd, int nblk, float* dW, float* db, cudaStream_t s);
+int wgrad_blocks(int nsm, int cx, int cd);  // most blocks of a pass (rows of part and part_b)
+int wgrad(const WgradArgs& a, int cx, int cd, int nsm, float* dW, float* db, cudaStream_t s);
 int pack(const PackArgs& a, int fp64, int nsm, cudaStream_t s);
 int loss(const LossArgs& a, int nblk, double* out, cudaStream_t s);
 int adam(float* p, const float* g, float* m, float* v, int64_t n, double lr, int64_t step, cudaStream_t s);
