@@ -1,6 +1,7 @@
-"""Weight gradients of the closure with fewer tiles than blocks, with exactly
-one round of them, and with rounds that end unevenly (the tiles of a block
-alternate between two slots)."""
+"""Gradients of the closure with fewer tiles than blocks, with exactly one round
+of them, and with rounds that end unevenly (the tiles of a block alternate
+between two slots); on 64-site rows also the tensor-memory convolutions with
+runs of planes that cross columns and that are longer than a column."""
 from __future__ import annotations
 
 import numpy as np
@@ -14,7 +15,8 @@ pytestmark = pytest.mark.gpu
 
 
 # (sites, samples): 16 x 8 sites of one plane are a tile
-@pytest.mark.parametrize("shape,idx", [((16, 8, 1), [0]), ((48, 24, 17), [1]), ((64, 16, 19), [1, 0, 1])])
+@pytest.mark.parametrize("shape,idx", [((16, 8, 1), [0]), ((48, 24, 17), [1]), ((64, 16, 19), [1, 0, 1]),
+                                       ((64, 64, 3), [0, 1, 1, 0, 1, 0, 0, 1, 1, 0, 1])])
 def test_gradients_over_uneven_rounds(engine, shape, idx):
     host, buf = _dataset(engine, shape, 2, 21)
     net, p, norm = _net(engine, 23)
