@@ -107,10 +107,10 @@ __global__ void __launch_bounds__(256) energy_kernel(EnergyArgs a) {
 // FP64 finite-difference lattices: red[0..3], red[4] = -sum phi L phi, red[5] = sum
 // of the squared differences and, with strains, red[6] = sum w pu^2, red[7] =
 // -sum w u L u (w = 2 off the diagonal), over planes [zlo, zhi).  A thread
-// marches along z with the centre and the face- and corner-neighbour sums of
-// three planes in registers, so a plane is read once (9 values instead of 27
-// per site); each pair of neighbours enters the squared differences once, at
-// its lower site, for both.
+// marches along z and reads a plane once (9 values instead of 27 per site); per
+// array it keeps what the last plane adds to its neighbours and the Laplacian in
+// progress, as the FP64 steps do.  Each pair of neighbours enters the squared
+// differences once, at its lower site, for both.  Bound by the FP64 pipe.
 template <int NF, bool GW, bool SEVEN>
 __global__ void __launch_bounds__(128) fd_energy_kernel(EnergyArgs a, int zlo, int zhi, int zc) {
   using R = double;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(128) fd_energy_kernel(EnergyArgs a, int zlo, i
     auto base = [&](int c) {
       return c < NF ? static_cast<const R*>(a.phi) + c * N : static_cast<const R*>(a.u) + (c - NF) * N;
     };
-    R wc[NC][3], w1[NC][3], w2[NC][3];
+    R wc[NC][3], tz[NC], la[NC], ln[NC];  // centres; neighbour term; Laplacian of planes z, z + 1
     R e1[NF], e2[NF];  // in-plane squared differences of the middle plane's pairs
     // plane z into slot k; diffs of the pairs (z-1, z) and inside z for the fields
     auto load = [&](int z, int k, bool pairs) {
@@ -147,8 +147,13 @@ __global__ void __launch_bounds__(128) fd_energy_kernel(EnergyArgs a, int zlo, i
           }
         }
         wc[c][k] = v[1][1];
-        w1[c][k] = (v[1][0] + v[1][2]) + (v[0][1] + v[2][1]);
-        if (!SEVEN) w2[c][k] = (v[0][0] + v[0][2]) + (v[2][0] + v[2][2]);
+        const R s1 = (v[1][0] + v[1][2]) + (v[0][1] + v[2][1]);
+        const R s2 = SEVEN ? R(0) : (v[0][0] + v[0][2]) + (v[2][0] + v[2][2]);
+        const R t = SEVEN ? c1 * v[1][1] : c1 * v[1][1] + c2 * s1 + c3 * s2;
+        if (k == 2) la[c] += t;  // plane z - 1 is complete
+        if (k > 0) ln[c] = SEVEN ? tz[c] + c0 * v[1][1] + c1 * s1 : tz[c] + c0 * v[1][1] + c1 * s1 + c2 * s2;
+        if (k == 1) la[c] = ln[c];
+        tz[c] = t;
         if (c < NF) {
           auto sq = [](R p, R q) { const R d = p - q; return d * d; };
           if (pairs) {  // with plane z - 1 (slot k - 1)
@@ -172,20 +177,13 @@ __global__ void __launch_bounds__(128) fd_energy_kernel(EnergyArgs a, int zlo, i
     for (int z = z0; z < z1; ++z) {
       const int64_t t = (int64_t)z * plane + row[1] + x;
       load(z + 1, 2, true);
-      R lap[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const R r1 = w1[c][1] + (wc[c][0] + wc[c][2]);
-        lap[c] = c0 * wc[c][1] + c1 * r1;
-        if (!SEVEN) lap[c] += c2 * (w2[c][1] + (w1[c][0] + w1[c][2])) + c3 * (w2[c][0] + w2[c][2]);
-      }
       R f[NF], ke = R(0);
 #pragma unroll
       for (int l = 0; l < NF; ++l) {
         f[l] = wc[l][1];
         const R p = static_cast<const R*>(a.pi)[l * N + t];
         ke += p * p;
-        s[4].add(-f[l] * lap[l]);
+        s[4].add(-f[l] * la[l]);
       }
       s[0].add(ke);
       s[1].add(model_v<R, NF>(a.model, f));
@@ -196,20 +194,17 @@ __global__ void __launch_bounds__(128) fd_energy_kernel(EnergyArgs a, int zlo, i
 #pragma unroll
         for (int g = 0; g < 6; ++g) {
           const R p = static_cast<const R*>(a.pu)[g * N + t];
-          if (g < 3) { d += p * p; dl -= wc[NF + g][1] * lap[NF + g]; }
-          else { o += p * p; ol -= wc[NF + g][1] * lap[NF + g]; }
+          if (g < 3) { d += p * p; dl -= wc[NF + g][1] * la[NF + g]; }
+          else { o += p * p; ol -= wc[NF + g][1] * la[NF + g]; }
         }
         s[6].add(d + (o + o));
         s[7].add(dl + (ol + ol));
       }
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          wc[c][k] = wc[c][k + 1];
-          w1[c][k] = w1[c][k + 1];
-          w2[c][k] = w2[c][k + 1];
-        }
+        wc[c][0] = wc[c][1];
+        wc[c][1] = wc[c][2];
+        la[c] = ln[c];
       }
     }
   }
