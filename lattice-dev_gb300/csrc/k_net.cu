@@ -759,15 +759,19 @@ int out_conv_go(const ConvArgs& a, int nsm, cudaStream_t s) {
   return e == cudaSuccess ? LAT_OK : cuda_fail(e, "output conv launch");
 }
 
+bool tc_off() {
+  static const bool off = [] {
+    const char* v = getenv("LAT_NO_TCGEN05");
+    return v && v[0] && v[0] != '0';
+  }();
+  return off;
+}
+
 }  // namespace
 
 int conv(const ConvArgs& a, int ca, int cb, int epi, int nsm, cudaStream_t s) {
   if (a.nx % TX || a.ny % TY || a.nz < 1) return set_error(LAT_ERR_ARG, "closure lattice: nx % 16, ny % 8");
-  static const bool no_tc = [] {
-    const char* v = getenv("LAT_NO_TCGEN05");
-    return v && v[0] && v[0] != '0';
-  }();
-  if (!no_tc && a.err && conv_tc_ok(ca, cb, epi, a.nx, a.ny)) return conv_tc(a, ca, epi, nsm, a.err, s);
+  if (!tc_off() && a.err && conv_tc_ok(ca, cb, epi, a.nx, a.ny)) return conv_tc(a, ca, epi, nsm, a.err, s);
   const bool sz = a.zout != nullptr;
   if (ca == 8 && cb == 32 && epi == EPI_GELU) return sz ? conv_go<8, 32, EPI_GELU, true>(a, nsm, s)
                                                         : conv_go<8, 32, EPI_GELU, false>(a, nsm, s);
@@ -784,7 +788,9 @@ int conv(const ConvArgs& a, int ca, int cb, int epi, int nsm, cudaStream_t s) {
   return set_error(LAT_ERR_UNSUPPORTED, "conv shape");
 }
 
-// Blocks of a weight-gradient pass: what fits an SM, one for 32 x 32 channels
+// Weight gradients run on tcgen05 where a layer has 32 input channels and rows
+// are multiples of 32 (91 against 222 us, 44 against 107), else on mma.sync.
+// Blocks of an mma.sync pass: what fits an SM, one for 32 x 32 channels
 // (registers), two for 32 x 8 (90 KB of shared memory each) and three for
 // 8 x 32, which waits on its fragments and barriers otherwise.
 int wgrad_blocks(int nsm, int cx, int cd) { return nsm * (cx == 8 ? 3 : (cd == 8 ? 2 : 1)); }
@@ -793,7 +799,7 @@ int wgrad(const WgradArgs& a, int cx, int cd, int nsm, float* dW, float* db, cud
   if (a.nx % TX || a.ny % TY) return set_error(LAT_ERR_ARG, "closure lattice: nx % 16, ny % 8");
   cudaError_t e;
   const int64_t ntiles = (int64_t)(a.nx / TX) * (a.ny / TY) * a.nz * a.nlat;
-  const int nblk = (int)std::min<int64_t>(ntiles, wgrad_blocks(nsm, cx, cd));
+  int nblk = (int)std::min<int64_t>(ntiles, wgrad_blocks(nsm, cx, cd));
   auto go = [&](auto kern, int CX, int CD, int WM) -> int {
     const size_t smem = (size_t)(HSITES * (CX == 32 ? 40 : 8) + TSITES * (CD == 32 ? 40 : 8)) * 2 * 2;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -804,7 +810,8 @@ int wgrad(const WgradArgs& a, int cx, int cd, int nsm, float* dW, float* db, cud
     return e == cudaSuccess ? LAT_OK : cuda_fail(e, "wgrad launch");
   };
   int st;
-  if (cx == 32 && cd == 8) st = go(wgrad_kernel<32, 8, 2>, 32, 8, 2);
+  if (!tc_off() && a.err && wgrad_tc_ok(cx, cd, a.nx, a.ny)) st = wgrad_tc(a, cd, nsm, &nblk, s);
+  else if (cx == 32 && cd == 8) st = go(wgrad_kernel<32, 8, 2>, 32, 8, 2);
   else if (cx == 32 && cd == 32) st = go(wgrad_kernel<32, 32, 1>, 32, 32, 1);
   else if (cx == 8 && cd == 32) st = go(wgrad_kernel<8, 32, 2>, 8, 32, 2);
   else return set_error(LAT_ERR_UNSUPPORTED, "wgrad shape");

@@ -179,6 +179,7 @@ int loss_and_grad(lat_net_s* n, const float* data, int64_t stride, int nidx, int
   la.part = n->lpart;
   NRET(lat::net::loss(la, 2 * n->nsm, n->lsum, s));
   WgradArgs w{};
+  w.err = n->err;
   w.nx = nx; w.ny = ny; w.nz = nz; w.nlat = nidx;
   w.part = n->part;
   w.part_b = n->part_b;

@@ -38,6 +38,7 @@ struct WgradArgs {
   const __nv_bfloat16* d;  // [nlat][N][CD] gradient at the layer's pre-activation
   float* part;             // [nblk][27][CX][CD]
   float* part_b;           // [nblk][CD]
+  int* err;                // device error word (bounded waits of the tensor-memory kernel)
 };
 
 struct PackArgs {
@@ -94,6 +95,9 @@ int conv(const ConvArgs& a, int ca, int cb, int epi, int nsm, cudaStream_t s);
 bool conv_tc_ok(int ca, int cb, int epi, int nx, int ny);
 int conv_tc(const ConvArgs& a, int ca, int epi, int nsm, int* err, cudaStream_t s);
 int wgrad_blocks(int nsm, int cx, int cd);  // most blocks of a pass (rows of part and part_b)
+// weight gradients of layers with 32 input channels on tcgen05 (k_wgrad_tc.cu)
+bool wgrad_tc_ok(int cx, int cd, int nx, int ny);
+int wgrad_tc(const WgradArgs& a, int cd, int nsm, int* nblk, cudaStream_t s);
 int wgrad(const WgradArgs& a, int cx, int cd, int nsm, float* dW, float* db, cudaStream_t s);
 int pack(const PackArgs& a, int fp64, int nsm, cudaStream_t s);
 int loss(const LossArgs& a, int nblk, double* out, cudaStream_t s);

@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 
 # (sites, samples): 16 x 8 sites of one plane are a tile
-@pytest.mark.parametrize("shape,idx", [((16, 8, 1), [0]), ((48, 24, 17), [1]), ((64, 16, 19), [1, 0, 1]),
+@pytest.mark.parametrize("shape,idx", [((16, 8, 1), [0]), ((48, 24, 17), [1]), ((32, 8, 1), [1]), ((96, 24, 2), [0, 1]), ((64, 16, 19), [1, 0, 1]),
                                        ((64, 64, 3), [0, 1, 1, 0, 1, 0, 0, 1, 1, 0, 1])])
 def test_gradients_over_uneven_rounds(engine, shape, idx):
     host, buf = _dataset(engine, shape, 2, 21)
