@@ -1477,11 +1477,6 @@ int lat_create(lat_t** out, const lat_config* cfg) {
   }
   if ((st = make_fx_tables(h))) return bail(st);
   if (spectral(h) && cfg->spectral_impl == LAT_SPEC_IMPL_AUTO) h->sep = auto_separable(h);
-  h->ev_pool.resize(4096);
-  for (auto& ev : h->ev_pool) {
-    cudaEventCreate(&ev.a);
-    cudaEventCreate(&ev.b);
-  }
   if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return bail(cuda_fail(e, "create sync"));
   h->use_graphs = !getenv_flag("LAT_NO_GRAPHS");
   *out = h;
@@ -2068,6 +2063,21 @@ int lat_checkpoint_read(lat_t* h, const char* dir, double* time, int32_t* frame)
 
 int lat_timing_enable(lat_t* h, int32_t on) {
   if (!h) return set_error(LAT_ERR_ARG, "null handle");
+  if (on && h->ev_pool.empty()) {  // the launch timer's events, with its first use
+    ApiGuard g(h);
+    h->ev_pool.reserve(4096);
+    while (h->ev_pool.size() < 4096) {
+      lat_s::Ev ev = {};
+      cudaError_t e = cudaEventCreate(&ev.a);
+      if (e == cudaSuccess && (e = cudaEventCreate(&ev.b)) != cudaSuccess) cudaEventDestroy(ev.a);
+      if (e != cudaSuccess) {
+        for (auto& v : h->ev_pool) { cudaEventDestroy(v.a); cudaEventDestroy(v.b); }
+        h->ev_pool.clear();
+        return cuda_fail(e, "timing events");
+      }
+      h->ev_pool.push_back(ev);
+    }
+  }
   h->timing = on != 0;
   return LAT_OK;
 }
