@@ -33,8 +33,8 @@
 // instruction itself is predicated on the elected lane.  Four 64^3 lattices,
 // 32 -> 32 with z stored: 134 us as it was, 115 with N = 96, 91 with the
 // converged warp, 89-93 with copies and epilogue in warps of their own (one
-// 64^3 lattice: 38.7 -> 33); 4 -> 32: 69 -> 56.  What is left: MMAs alone 58,
-// stores and copies 50 each.
+// 64^3 lattice: 38.7 -> 33; 128^3: 234 -> 145, 800 TFLOP/s); 4 -> 32: 69 -> 56.  What
+// is left: MMAs alone 58, stores and copies 50 each.
 //
 // Every wait is bounded: a warp that gives up raises a shared abort flag that
 // the whole block reads after its next barrier; the block then sets the error

@@ -281,7 +281,8 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_tc_kernel(WgradArgs a, int*
 }  // namespace
 
 bool wgrad_tc_ok(int cx, int cd, int nx, int ny) {
-  return cx == 32 && (cd == 32 || cd == 8) && nx % WX == 0 && ny % WY == 0;
+  // a plane's offsets are 32-bit
+  return cx == 32 && (cd == 32 || cd == 8) && nx % WX == 0 && ny % WY == 0 && (int64_t)nx * ny < (1LL << 26);
 }
 
 int wgrad_tc(const WgradArgs& a, int cd, int nsm, int* nblk, cudaStream_t s) {
