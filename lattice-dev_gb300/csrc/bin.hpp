@@ -4,10 +4,9 @@
 #include <vector>
 
 #include "engine.hpp"
+#include "sizes.hpp"
 
 namespace lat {
-
-constexpr int kMaxBins = 2048;
 
 struct BinArgs {
   int nx, ny, nz;

@@ -84,9 +84,11 @@ __global__ void __launch_bounds__(256) bin_kernel(BinArgs a) {
   const int hx = a.nx / 2 + 1, hy = a.ny / 2 + 1, hz = a.nz / 2 + 1;
   const C* F1 = static_cast<const C*>(a.F[0]);
   const C* F2 = static_cast<const C*>(a.F[1]);
-  const int nrow = hy * hz;
+  const int nrow = hy * hz, xend = min(hx, nb);
   for (int row = blockIdx.x * nw + warp; row < nrow; row += gridDim.x * nw) {
-    const int jj = row % hy, kk = row / hy, r2 = jj * jj + kk * kk;
+    const int jj = row % hy, kk = row / hy;
+    if (jj >= nb || kk >= nb) continue;  // beyond the last shell, as the x from nb on: |n|^2 stays below 3 nb^2
+    const int r2 = jj * jj + kk * kk;
     const int my = (jj == 0 || 2 * jj == a.ny) ? 1 : 2, mz = (kk == 0 || 2 * kk == a.nz) ? 1 : 2;
     size_t at[4];  // the rows (+-y, +-z)
 #pragma unroll
@@ -94,9 +96,9 @@ __global__ void __launch_bounds__(256) bin_kernel(BinArgs a) {
       const int y = my == 2 && (r & 1) ? a.ny - jj : jj, z = (my == 2 ? r >> 1 : r) ? a.nz - kk : kk;
       at[r] = ((size_t)z * a.ny + y) * hx;
     }
-    for (int x0 = 0; x0 < hx; x0 += 32) {
+    for (int x0 = 0; x0 < xend; x0 += 32) {
       const int x = x0 + lane;
-      const bool on = x < hx;
+      const bool on = x < xend;
       const int m2 = r2 + x * x, l = on ? isqrt_exact(m2) : 0x40000000 + lane;
       double v = 0.0, vi = 0.0;
       if constexpr (KIND == BIN_GW) {
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(256) bin_kernel(BinArgs a) {
       }
       double s[NS];
       if constexpr (KIND == BIN_POWER || KIND == BIN_CROSS) {
-        const double2 c = on ? __ldg(a.wtab + m2) : make_double2(0.0, 0.0);
+        const double2 c = on && l < nb ? __ldg(a.wtab + m2) : make_double2(0.0, 0.0);  // m2 < nb^2
         s[0] = c.x * v;
         s[1] = c.y * v;
         if constexpr (KIND == BIN_CROSS) {
@@ -203,14 +205,15 @@ __global__ void bin_weight_kernel(double2* wtab, int n) {
     wtab[m2] = make_double2(__dmul_rn(e0, e0), __dmul_rn(e1, e1));
   }
 }
-// modes of the full spectrum at every |n|^2
-__global__ void bin_count_kernel(int* cnt, int nx, int ny, int nz) {
+// modes of the full spectrum at every |n|^2 below n
+__global__ void bin_count_kernel(int* cnt, int n, int nx, int ny, int nz) {
   const int hx = nx / 2 + 1, hy = ny / 2 + 1, hz = nz / 2 + 1;
   const long long tot = (long long)hx * hy * hz;
   auto mult = [](int i, int n) { return i == 0 || 2 * i == n ? 1 : 2; };
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (long long)gridDim.x * blockDim.x) {
     const int x = (int)(t % hx), y = (int)(t / hx % hy), z = (int)(t / hx / hy);
-    atomicAdd(cnt + x * x + y * y + z * z, mult(x, nx) * mult(y, ny) * mult(z, nz));
+    const long long m2 = (long long)x * x + (long long)y * y + (long long)z * z;
+    if (m2 < n) atomicAdd(cnt + m2, mult(x, nx) * mult(y, ny) * mult(z, nz));
   }
 }
 // W[l]: two-bin weight sums, W[nb + l]: counts; one warp per shell
@@ -276,9 +279,9 @@ int BinPlan::make(int nx_, int ny_, int nz_, int nsm_, cudaStream_t s) {
   nsm = nsm_;
   // one allocation: weights, sines, output, counter, and the partial sums,
   // whose space first holds the counts and the weight sums
-  const int n = (nx / 2) * (nx / 2) + (ny / 2) * (ny / 2) + (nz / 2) * (nz / 2) + 1;
+  const int n = (int)bin_table_size(nx, ny, nz);
   const size_t ns = (size_t)(nx / 2 + 1) + ny + nz, no = (size_t)4 * kMaxBins;
-  const size_t np = std::max<size_t>(no * 2 * nsm, 2 * kMaxBins + (size_t)n);
+  const size_t np = std::max<size_t>(no * 2 * nsm, 2 * kMaxBins + ((size_t)n + 1) / 2);
   double* mem = nullptr;
   cudaError_t e = cudaMalloc(&mem, sizeof(double) * (2 * (size_t)n + ns + no + 8 + np));
   if (e != cudaSuccess) return set_error(LAT_ERR_ALLOC, std::string("spectrum tables: ") + cudaGetErrorString(e));
@@ -296,7 +299,7 @@ int BinPlan::make(int nx_, int ny_, int nz_, int nsm_, cudaStream_t s) {
     const long long oct = (long long)(nx / 2 + 1) * (ny / 2 + 1) * (nz / 2 + 1);
     bin_weight_kernel<<<std::min((n + 255) / 256, 4 * nsm), 256, 0, s>>>(wtab, n);
     bin_sin_kernel<<<8, 128, 0, s>>>(sins, nx, ny, nz);
-    bin_count_kernel<<<(int)std::min<long long>((oct + 255) / 256, 8 * nsm), 256, 0, s>>>(cnt, nx, ny, nz);
+    bin_count_kernel<<<(int)std::min<long long>((oct + 255) / 256, 8 * nsm), 256, 0, s>>>(cnt, n, nx, ny, nz);
     bin_sum_kernel<<<kMaxBins / 8, 256, 0, s>>>(cnt, wtab, n, kMaxBins, W);
     if (g_launch_counter) *g_launch_counter += 4;
     e = cudaGetLastError();
