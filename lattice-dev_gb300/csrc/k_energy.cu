@@ -454,23 +454,24 @@ __global__ void __launch_bounds__(256) parseval_kernel(const C* F, int nx, int n
 }
 
 // ------------------------------------------------------------- ensembles
-// Every run of an ensemble in one launch: blockIdx.y is the run, its first
-// chunks(run) blocks share it; the last to arrive leaves the run's sums in
-// out[run * 8 ..] in block order.  MODE 0: sum pi^2, V, phi; 1: Parseval sum.
+// Every run of an ensemble in one launch: blockIdx.x is the run (along y a grid
+// holds 65535 blocks, an ensemble may hold more runs), its first run.blocks
+// blocks share it; the last to arrive leaves the run's sums in out[run * 8 ..]
+// in block order.  MODE 0: sum pi^2, V, phi; 1: Parseval sum.
 template <typename R, typename C, int MODE>
 __global__ void __launch_bounds__(256) ens_energy_kernel(EnsEnergyArgs a) {
   constexpr int NV = MODE == 0 ? 3 : 1;
   __shared__ int am_last;
-  const EnsEnergyRun run = a.runs[blockIdx.y];
+  const EnsEnergyRun run = a.runs[blockIdx.x];
   const int n = run.n, nblk = run.blocks;
-  if ((int)blockIdx.x >= nblk) return;
+  if ((int)blockIdx.y >= nblk) return;
   using Acc = typename AccOf<R>::type;
   double s[NV];
   if (MODE == 0) {
     Acc q[4];
     const int64_t N = (int64_t)n * n * n;
     const R *phi = static_cast<const R*>(a.phi) + run.site, *pi = static_cast<const R*>(a.pi) + run.site;
-    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)nblk * blockDim.x;
+    const int64_t t0 = (int64_t)blockIdx.y * blockDim.x + threadIdx.x, step = (int64_t)nblk * blockDim.x;
     if (N % 4 == 0 && run.site % 4 == 0) quad_sums<R, 1>(phi, pi, N, t0, N / 4, step, a.model, q);
     else site_sums<R, 1>(phi, pi, N, t0, N, step, a.model, q);
     const typename Acc::Red v[3] = {q[0].red(), q[1].red(), q[2].red()};
@@ -479,7 +480,7 @@ __global__ void __launch_bounds__(256) ens_energy_kernel(EnsEnergyArgs a) {
     for (int i = 0; i < NV; ++i) s[i] = b[i];
   } else {
     Acc acc;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarp = (nblk * blockDim.x) >> 5;
+    const int warp = (blockIdx.y * blockDim.x + threadIdx.x) >> 5, nwarp = (nblk * blockDim.x) >> 5;
     parseval_rows<R>(static_cast<const C*>(a.Fk) + run.fk, n, n, n, (R)run.dk2, run.dk2, run.dk2, warp, nwarp,
                      threadIdx.x & 31, acc);
     const typename Acc::Red v[1] = {acc.red()};
@@ -487,11 +488,11 @@ __global__ void __launch_bounds__(256) ens_energy_kernel(EnsEnergyArgs a) {
     block_sums<1>(v, b);
     s[0] = b[0];
   }
-  double* part = a.partials + (size_t)blockIdx.y * a.max_blocks * 4;
+  double* part = a.partials + (size_t)blockIdx.x * a.max_blocks * 4;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NV; ++i) part[(size_t)blockIdx.x * NV + i] = s[i];
+    for (int i = 0; i < NV; ++i) part[(size_t)blockIdx.y * NV + i] = s[i];
     __threadfence();
-    am_last = atomicAdd(a.counters + blockIdx.y, 1u) == (unsigned int)nblk - 1u;
+    am_last = atomicAdd(a.counters + blockIdx.x, 1u) == (unsigned int)nblk - 1u;
   }
   __syncthreads();
   if (!am_last) return;
@@ -499,8 +500,8 @@ __global__ void __launch_bounds__(256) ens_energy_kernel(EnsEnergyArgs a) {
   double tot[NV];
   row_sums<NV>(part, nblk, tot);
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NV; ++i) a.out[(size_t)blockIdx.y * 8 + (MODE == 0 ? i : 4)] = tot[i];
-    a.counters[blockIdx.y] = 0u;
+    for (int i = 0; i < NV; ++i) a.out[(size_t)blockIdx.x * 8 + (MODE == 0 ? i : 4)] = tot[i];
+    a.counters[blockIdx.x] = 0u;
   }
 }
 
@@ -525,7 +526,7 @@ int launch_parseval(const void* Fk, int nx, int ny, int nz, int nf, double dkx2,
 }
 
 int launch_ens_energies(const EnsEnergyArgs& a, int nruns, int parseval, int precision, cudaStream_t s) {
-  const dim3 grid(a.max_blocks, nruns);
+  const dim3 grid(nruns, a.max_blocks);  // at most 64 blocks a run
   if (precision == LAT_FP64) {
     if (parseval) ens_energy_kernel<double, double2, 1><<<grid, 256, 0, s>>>(a);
     else ens_energy_kernel<double, double2, 0><<<grid, 256, 0, s>>>(a);
