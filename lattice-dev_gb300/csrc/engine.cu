@@ -255,31 +255,6 @@ bool auto_separable(const lat_s* h) {
   return h->fx_ok && (h->nf == 2 || h->N > 32768) && !getenv_flag("LAT_NO_SEPARABLE");
 }
 
-// Tile of the stencil passes before any autotuning: 4 rows, and the chunk of
-// planes with the least estimated time: blocks share the SMs' throughput, so
-// the busiest SM's blocks times their planes (one block re-reads and re-sums
-// about half a plane in FP64, most of one in FP32), plus the latency of a
-// block's own chain where blocks are few.  Against 8 rows and 32 planes for
-// every lattice, a leapfrog step: 32^3 7-point FP64 48.4 -> 3.9 us (tuned:
-// 3.9), 64^3 48.4 -> 11.9 (10.9), 50 x 40 x 30 GW FP32 47.7 -> 6.1 (6.1), 144 x
-// 100 x 90 GW FP64 725 -> 470 (462), 256^3 GW FP32 382 -> 379 (376).
-void fd_default_tile(lat_s* h) {
-  const bool two = h->prec != LAT_FP64 && h->nx % 64 == 0;  // two x-sites per thread
-  const int cols = (h->nx + (two ? 63 : 31)) / (two ? 64 : 32) * ((h->ny + 3) / 4);
-  const double halo = h->prec == LAT_FP64 ? 0.5 : 0.8;
-  double best = 1e300;
-  h->fd_ty = 4;
-  for (int zc = 2; zc <= std::max(2, std::min(64, h->nz)); ++zc) {
-    const int64_t blocks = (int64_t)cols * ((h->nz + zc - 1) / zc);
-    const int64_t busiest = (blocks + h->nsm - 1) / h->nsm, rounds = (blocks + 4 * h->nsm - 1) / (4 * h->nsm);
-    const double cost = busiest * (zc + halo) + 0.35 * rounds * (zc + 3);
-    if (cost < best) {
-      best = cost;
-      h->fd_zc = std::min(zc, h->nz);
-    }
-  }
-}
-
 ModelP model_of(const lat_s* h) {
   ModelP m;
   m.model = h->cfg.model;
@@ -1417,7 +1392,9 @@ int lat_create(lat_t** out, const lat_config* cfg) {
   if ((st = alloc((void**)&h->rb.partials, (size_t)maxb * 16 * sizeof(double)))) return bail(st);
   if ((st = alloc((void**)&h->rb.counter, 64))) return bail(st);
   if ((st = h->bins.make(h->nx, h->ny, h->nz, h->nsm, h->stream))) return bail(st);
-  fd_default_tile(h);
+  const FdTile tile = fd_default_tile(h->nx, h->ny, h->nz, h->prec == LAT_FP64, h->nsm);
+  h->fd_ty = tile.ty;
+  h->fd_zc = tile.zc;
 
   if ((st = make_plan(h, &h->p_r2c1, &h->have_r2c1, true, 1))) return bail(st);
   if ((st = make_plan(h, &h->p_c2r1, &h->have_c2r1, false, 1))) return bail(st);
@@ -2298,7 +2275,7 @@ int lat_autotune(lat_t* h, const char* cache_path) {
     for (int ty : {2, 4, 8, 16})
       for (int zc : {2, 4, 8, 16, 32, 64}) {  // short z-chunks: enough blocks on small lattices
         if (st != LAT_OK) break;
-        if (zc > h->nz && zc != 8) continue;
+        if ((zc > h->nz && zc != 8) || !fd_tile_fits(h->ny, h->nz, ty, zc)) continue;
         h->fd_ty = ty;
         h->fd_zc = std::min(zc, h->nz);
         float ms = 0;

@@ -119,7 +119,8 @@ __global__ void __launch_bounds__(128) fd_energy_kernel(EnergyArgs a, int zlo, i
   Acc s[8];
   const int nx = a.nx, ny = a.ny, nz = a.nz;
   const int64_t N = (int64_t)nx * ny * nz, plane = (int64_t)nx * ny;
-  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 4 + threadIdx.y;
+  const int gx = (nx + 31) / 32;  // tiles of 32 x 4 sites, row by row along the grid's x
+  const int x = (int)(blockIdx.x % gx) * 32 + threadIdx.x, y = (int)(blockIdx.x / gx) * 4 + threadIdx.y;
   const int z0 = zlo + blockIdx.z * zc, z1 = min(z0 + zc, zhi);
   if (x < nx && y < ny) {
     const int xm = x ? x - 1 : nx - 1, xp = x + 1 < nx ? x + 1 : 0;
@@ -233,7 +234,8 @@ __global__ void __launch_bounds__(128) fd_energy32_kernel(EnergyArgs a, int zlo,
   KSum s[8];
   const int nx = a.nx, ny = a.ny, nz = a.nz;
   const int64_t N = (int64_t)nx * ny * nz, plane = (int64_t)nx * ny;
-  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 4 + threadIdx.y;
+  const int gx = (nx + 31) / 32;  // tiles of 32 x 4 sites, row by row along the grid's x
+  const int x = (int)(blockIdx.x % gx) * 32 + threadIdx.x, y = (int)(blockIdx.x / gx) * 4 + threadIdx.y;
   const int z0 = zlo + blockIdx.z * zc, z1 = min(z0 + zc, zhi);
   if (x < nx && y < ny) {
     const int col[3] = {x ? x - 1 : nx - 1, x, x + 1 < nx ? x + 1 : 0};
@@ -381,7 +383,7 @@ int energy_go(const EnergyArgs& a, cudaStream_t s) {
   const int gx = (a.nx + 31) / 32, gy = (a.ny + 3) / 4;
   const int want = std::max(1, (8 * (a.grid / 4) + gx * gy - 1) / (gx * gy));
   const int zc = std::max(2, (zhi - zlo + want - 1) / want);
-  const dim3 grid(gx, gy, (zhi - zlo + zc - 1) / zc), block(32, 4);
+  const dim3 grid(gx * gy, 1, (zhi - zlo + zc - 1) / zc), block(32, 4);
 #define LAT_FD_ENERGY(GWV, SEV)                                                                          \
   do {                                                                                                  \
     if constexpr (sizeof(R) == 8) fd_energy_kernel<NF, GWV, SEV><<<grid, block, 0, s>>>(a, zlo, zhi, zc); \

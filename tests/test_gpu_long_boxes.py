@@ -1,7 +1,8 @@
 """Long thin and wide boxes: shapes whose longest side is far beyond the others.
 
 Spectra of sides beyond 4096 points, which hold |n|^2 past the last shell (2047),
-against numpy.  Counts and weights hold no data: they agree to rounding.  A bin's
+against numpy; stencil steps and energies of more rows or planes than a grid of four
+rows a block holds, against the same leapfrog in numpy.  Counts and weights hold no data: they agree to rounding.  A bin's
 modes carry the rounding of an FP64 transform, below 1e-11 of the mean power.
 """
 from __future__ import annotations
@@ -49,4 +50,52 @@ def test_spectra(engine, shape, nb):
     S, Wg = g.spectrum_bin(L.SPEC_FLD, 0, nb)
     assert np.array_equal(Wg, cnt)
     assert np.all(np.abs(S * np.maximum(cnt, 1) - np.bincount(l, w * F, nb)) <= 1e-11 * (np.bincount(l, w * F, nb) + tot * cnt))
+    g.close()
+
+
+def neighbours(g, lap):
+    """Sums over the 6 face and, with 27 points, 12 edge and 8 corner neighbours."""
+    n = lambda v, d: np.roll(v, 1, d) + np.roll(v, -1, d)  # noqa: E731
+    sx, sy = n(g, 2), n(g, 1)
+    r = [sx + sy + n(g, 0)]
+    if lap == L.LAP_FD27:
+        sxy = n(sx, 1)
+        r += [sxy + n(sx + sy, 0), n(sxy, 0)]
+    return r
+
+
+@pytest.mark.parametrize("prec,tol", [(L.FP64, 1e-12), (L.FP32_KAHAN, 2e-5)])
+@pytest.mark.parametrize("shape,lap", [((2, 262200, 2), L.LAP_FD7), ((2, 262200, 2), L.LAP_FD27),
+                                       ((3, 2, 140000), L.LAP_FD7), ((3, 2, 140000), L.LAP_FD27),
+                                       ((64, 262148, 2), L.LAP_FD27)])
+def test_stencil_step_and_energies(engine, shape, lap, prec, tol):
+    """Two leapfrog steps and the energies on the untuned tile.  FP64: sums of 27 terms of order one, a few
+    steps; FP32: the same to the format, energies as sums of FP32 terms."""
+    nx, ny, nz = shape
+    c = (-6.0, 1.0, 0.0, 0.0, 1.0) if lap == L.LAP_FD7 else (-128.0, 14.0, 3.0, 1.0, 30.0)
+    g = engine.Lattice(L.make_config(shape, nfld=1, length=1.0 * nx, laplacian=lap, precision=prec,
+                                     model=L.MODEL_PHI4, model_params=(1.0,)))
+    dt = 0.05
+    f, p = (v[0] for v in random_state((1, nz, ny, nx), seed=11, mean=0.5, amp=0.3))
+    g.set_state(f[None], p[None])
+    f, p = (v[0] for v in g.get_state())
+
+    def laplacian(v):
+        r = neighbours(v, lap)
+        return (c[0] * v + sum(w * s for w, s in zip(c[1:], r))) / c[4]
+
+    e = g.energies()
+    q = sum(w * (s2 - 2 * f * s1 + k * f * f) for w, s1, s2, k in
+            zip(c[1:], neighbours(f, lap), neighbours(f * f, lap), (6, 12, 8)))
+    want = {L.E_KE: 0.5 * np.mean(p * p), L.E_GE_LAP: -0.5 * np.mean(f * laplacian(f)),
+            L.E_GE_GRAD: 0.25 * np.mean(q) / c[4], L.E_PE: 0.25 * np.mean(f ** 4), L.E_MEAN0: np.mean(f)}
+    for i, v in want.items():
+        assert abs(e[i] - v) <= tol * abs(v), i
+    for s in range(2):
+        f = f + dt * p * (0.5 if s == 0 else 1.0)
+        p = p + dt * (laplacian(f) - f ** 3)
+    f = f + 0.5 * dt * p
+    g.symp(2, dt, 2)
+    F, P = (v[0] for v in g.get_state())
+    assert np.max(np.abs(F - f)) <= tol and np.max(np.abs(P - p)) <= tol
     g.close()

@@ -33,3 +33,18 @@ def test_shell_tables(lib, shape):
     top = sum((s // 2) ** 2 for s in shape)
     assert n == min(top + 1, BINS ** 2)
     assert 24 * n <= 101 * 2 ** 20  # weights and counts
+
+
+@pytest.mark.parametrize("fp64", [0, 1])
+@pytest.mark.parametrize("shape", SHAPES + [(2, 262140, 2), (2, 262141, 2), (64, 262200, 3), (2, 524280, 4),
+                                            (2, 2, 4194240), (2, 4, 4194300)])
+def test_default_stencil_tile(lib, shape, fp64):
+    """The untuned stencil pass of every lattice has a grid: rows of blocks along y and chunks along z
+    are at most 65535 up to 524280 rows (8 a block, as far as an untuned pass ever went; 16 beyond)."""
+    nx, ny, nz = shape
+    out = (C.c_int * 3)()
+    lib.fd_tile(nx, ny, nz, fp64, 152, out)
+    ty, zc, fits = out
+    assert 1 <= zc <= nz and ty == (4 if ny <= 4 * 65535 else 8 if ny <= 8 * 65535 else 16)
+    assert -(-nz // zc) <= 65535
+    assert bool(fits) == (-(-ny // ty) <= 65535)
