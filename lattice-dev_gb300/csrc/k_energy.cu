@@ -405,16 +405,16 @@ int energy_go(const EnergyArgs& a, cudaStream_t s) {
 
 // ------------------------------------------------------------- Parseval
 // Sum over a half spectrum of w k^2 |F_k|^2, w = 2 for the modes whose
-// conjugate partner is not stored.  A warp adds the (up to four) rows (+-y,
-// +-z), which share k_y^2 + k_z^2, before two multiply-adds; terms in the
-// field precision, compensated FP32 or FP64 sums per lane.
+// conjugate partner is not stored.  A warp takes the (up to four) rows (+-y,
+// +-z), which share k_y^2 + k_z^2, together.  FP64 adds them before two
+// multiply-adds; in FP32 every mode's term enters the compensated sum by itself.
 template <typename R, typename C, typename Acc>
 __device__ __forceinline__ void parseval_rows(const C* F, int nx, int ny, int nz, R dkx2, double dky2, double dkz2,
                                               int row0, int step, int lane, Acc& acc) {
   const int hx = nx / 2 + 1, hy = ny / 2 + 1, hz = nz / 2 + 1;
   for (int row = row0; row < hy * hz; row += step) {
     const int jj = row % hy, kk = row / hy;
-    const R kyz = (R)((double)(jj * jj) * dky2 + (double)(kk * kk) * dkz2);
+    const R kyz = (R)((double)((int64_t)jj * jj) * dky2 + (double)((int64_t)kk * kk) * dkz2);
     const int my = (jj == 0 || 2 * jj == ny) ? 1 : 2, mz = (kk == 0 || 2 * kk == nz) ? 1 : 2;
     size_t at[4];
 #pragma unroll
@@ -430,12 +430,21 @@ __device__ __forceinline__ void parseval_rows(const C* F, int nx, int ny, int nz
         v[r] = C{0, 0};
         if (r < my * mz) v[r] = F[at[r] + x];
       }
-      R t = R(0);
+      const bool twice = x != 0 && 2 * x != nx;
+      R k2 = (R)((int64_t)x * x) * dkx2 + kyz;
+      if constexpr (sizeof(R) == sizeof(double)) {
+        R t = R(0);
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-        if (r < my * mz) t += v[r].x * v[r].x + v[r].y * v[r].y;
-      if (x != 0 && 2 * x != nx) t += t;
-      acc.add(((R)(x * x) * dkx2 + kyz) * t);
+        for (int r = 0; r < 4; ++r)
+          if (r < my * mz) t += v[r].x * v[r].x + v[r].y * v[r].y;
+        if (twice) t += t;
+        acc.add(k2 * t);
+      } else {
+        if (twice) k2 += k2;
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (r < my * mz) acc.add(k2 * (v[r].x * v[r].x + v[r].y * v[r].y));
+      }
     }
   }
 }
