@@ -250,16 +250,18 @@ __global__ void bin_sin_kernel(double* s, int nx, int ny, int nz) {
 template <int KIND>
 int bin_go(BinArgs a, int precision, int nsm, cudaStream_t s) {
   const size_t per = (size_t)Sums<KIND>::NS * a.nbins * sizeof(double);  // one warp's bins
+  constexpr size_t most = 96 * 1024;
   int warps = 8;
-  while (warps > 1 && warps * per > 96 * 1024) warps /= 2;
+  while (warps > 1 && warps * per > most) warps /= 2;
   const size_t smem = warps * per;
   auto k64 = bin_kernel<KIND, double2>;
   auto k32 = bin_kernel<KIND, float2>;
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(precision == LAT_FP64 ? k64 : k32,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_fail(e, "binning smem attribute");
-  }
+  // the limit belongs to the kernel, not to the call: always the largest size,
+  // which another thread's call may be about to launch with (and always, as the
+  // static shared memory counts towards the default 48 KB too)
+  const cudaError_t es = cudaFuncSetAttribute(precision == LAT_FP64 ? k64 : k32,
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+  if (es != cudaSuccess) return cuda_fail(es, "binning smem attribute");
   const int rows = (a.ny / 2 + 1) * (a.nz / 2 + 1);
   const int grid = std::min(2 * nsm, (rows + warps - 1) / warps);
   if (precision == LAT_FP64) k64<<<grid, 32 * warps, smem, s>>>(a);
