@@ -653,6 +653,19 @@ __global__ void __launch_bounds__(256) fd2_kernel(FdArgs a) {
   }
 }
 
+// The limit of dynamic shared memory belongs to the kernel, not to the call:
+// always that of the largest tile (16 rows of eight FP64 arrays), as another
+// thread's lattice may be about to launch a larger tile than this one's.  Below
+// 30 KB the default holds the tile and the reduction's static arrays.
+constexpr size_t kFdSmem = 120 * 1024;
+template <typename K>
+int fd_smem(K k, size_t smem) {
+  if (smem <= 30 * 1024) return LAT_OK;
+  if (smem > kFdSmem) return set_error(LAT_ERR_ARG, "FD tile too large");
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFdSmem);
+  return e == cudaSuccess ? LAT_OK : cuda_fail(e, "fd smem attribute");
+}
+
 template <bool KAHAN, int NF, bool GW, bool SEVEN, int MODE>
 int go2(const FdArgs& a, cudaStream_t s, int* nb) {
   constexpr int NC = NF + (GW ? 6 : 0);
@@ -663,10 +676,7 @@ int go2(const FdArgs& a, cudaStream_t s, int* nb) {
   dim3 grid(a.nx / 64, (a.ny + a.ty - 1) / a.ty, (nzc + a.zc - 1) / a.zc);
   const size_t smem = (size_t)3 * NC * kFd2Wd * (a.ty + 2) * sizeof(float);
   auto k = fd2_kernel<KAHAN, NF, GW, SEVEN, MODE>;
-  if (smem > 30 * 1024) {  // the reduction's static arrays count towards the 48 KB too
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_fail(e, "fd2 smem attribute");
-  }
+  if (const int st = fd_smem(k, smem)) return st;
   cudaError_t e = launch_pdl(k, grid, block, smem, s, a);
   if (e != cudaSuccess) return cuda_fail(e, "fd2 kernel launch");
   if (nb) *nb = grid.x * grid.y * grid.z;
@@ -689,10 +699,7 @@ int go(const FdArgs& a0, cudaStream_t s, int* nb) {
   if (a.ty < 1 || (!a.vec && 34 * (a.ty + 2) > kFdMaxSlots * 32 * a.ty))
     return set_error(LAT_ERR_ARG, "FD tile too narrow");
   auto k = fd_kernel<R, KAHAN, NF, GW, SEVEN, MODE>;
-  if (smem > 30 * 1024) {  // the reduction's static arrays count towards the 48 KB too
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_fail(e, "fd smem attribute");
-  }
+  if (const int st = fd_smem(k, smem)) return st;
   cudaError_t e = launch_pdl(k, grid, block, smem, s, a);
   if (e != cudaSuccess) return cuda_fail(e, "fd kernel launch");
   if (nb) *nb = grid.x * grid.y * grid.z;

@@ -6,6 +6,7 @@ sizes whose dynamic part alone just fills the default 48 KB.
 """
 from __future__ import annotations
 
+import re
 import threading
 
 import numpy as np
@@ -68,3 +69,28 @@ def test_bins_in_two_threads(engine):
         for _ in range(1500):
             h.spectrum(L.SPEC_FLD, 0, L.SPEC_WEIGHTED, 400)
     in_threads(many, fewer)
+
+
+def test_stencil_tiles_in_two_threads(engine, tmp_path, monkeypatch):
+    """Two lattices of one kernel whose tiles have eight and four rows (57 and 34 KB)."""
+    monkeypatch.setenv("LAT_NO_GRAPHS", "1")  # launches, not replays
+    kw = dict(model=L.MODEL_DOUBLE_WELL, model_params=(0.01,), gw=True, gw_coupling=1.0)
+    cache = tmp_path / "tune.jsonl"
+    first = lattice(engine, **kw)
+    first.autotune(cache)
+    line = cache.read_text()
+    gs = []
+    for ty in (8, 4):
+        c = tmp_path / ("tune%d.jsonl" % ty)
+        c.write_text(re.sub(r'"ty": \d+', '"ty": %d' % ty, line))
+        gs.append(lattice(engine, **kw))
+        gs[-1].autotune(c)
+        assert gs[-1].tuning()[1] == ty
+
+    def steps(g):
+        for _ in range(20):
+            g.symp(2, 1e-3, 200)
+            g.sync()
+    in_threads(lambda: steps(gs[0]), lambda: steps(gs[1]))
+    a, b = gs[0].get_state()[0], gs[1].get_state()[0]
+    assert np.max(np.abs(a - b)) <= 1e-9
