@@ -980,6 +980,17 @@ int ensure_stage(lat_s* h, size_t elems) {
   return LAT_OK;
 }
 
+// cuFFT takes real arrays from a 16-byte boundary on.  The second field of a
+// lattice with an odd number of sites (FP32: not a multiple of four) starts off
+// it; such an array is transformed from a copy in the stage.
+int fft_source(lat_s* h, const void** src) {
+  if (reinterpret_cast<uintptr_t>(*src) % 16 == 0) return LAT_OK;
+  RET(ensure_stage(h, (size_t)h->nf * h->N));
+  CK(cudaMemcpyAsync(h->stage, *src, (size_t)h->N * h->rsz, cudaMemcpyDeviceToDevice, h->stream));
+  *src = h->stage;
+  return LAT_OK;
+}
+
 // Host Fortran array (nfld, 1-lo:n+hi, ...) <-> unpadded AoS staging.
 int copy_aos(lat_s* h, double* host, int lo, int hi, bool to_device) {
   const int nf = h->nf;
@@ -1125,8 +1136,12 @@ int output_spectrum(lat_s* h, int what, int field, int slot, void** Fout, int* p
   RET(src_ptr(h, what, field, &src));
   if (h->prec == LAT_FP64) {
     void* F = (char*)h->Fk + (size_t)slot * h->M * h->csz;
-    if (h->fxr_ok) RET(fx_r2c(h, src, nullptr, static_cast<double2*>(F)));
-    else RET(fft_exec_r2c(h, h->p_r2c1, src, F));
+    if (h->fxr_ok) {
+      RET(fx_r2c(h, src, nullptr, static_cast<double2*>(F)));
+    } else {
+      RET(fft_source(h, &src));
+      RET(fft_exec_r2c(h, h->p_r2c1, src, F));
+    }
     *Fout = F;
     *prec = LAT_FP64;
     return LAT_OK;
@@ -1148,9 +1163,9 @@ int output_spectrum(lat_s* h, int what, int field, int slot, void** Fout, int* p
     CF(cufftSetStream(h->p_d2z1, h->stream));
     h->have_d2z1 = true;
   }
-  RET(ensure_stage(h, (size_t)std::max(h->nf, 2) * h->N));
+  RET(ensure_stage(h, (size_t)h->nf * h->N));
   const void* comp = (what == LAT_SPEC_FLD && h->fldc) ? (const char*)h->fldc + (size_t)field * h->N * h->rsz : nullptr;
-  double* tmp = h->stage + (size_t)slot * h->N;
+  double* tmp = h->stage;  // its start, for either slot: cuFFT refuses the odd places behind it
   RET(launch_to_fp64(src, comp, h->N, h->prec, tmp, h->stream));
   void* F = (double2*)h->Fk64 + (size_t)slot * h->M;
   {
@@ -1645,8 +1660,9 @@ int lat_laplacian(lat_t* h, int32_t field, double* out) {
   if (field < 0 || field >= h->nf) return set_error(LAT_ERR_ARG, "bad field index");
   ApiGuard g(h);
   RET(ensure_stage(h, (size_t)h->nf * h->N));
-  const char* src = (const char*)h->fld[h->cur] + (size_t)field * h->N * h->rsz;
+  const void* src = (const char*)h->fld[h->cur] + (size_t)field * h->N * h->rsz;
   if (spectral(h)) {
+    RET(fft_source(h, &src));
     RET(fft_exec_r2c(h, h->p_r2c1, src, h->Fk));
     KmulArgs k{};
     k.nx = h->nx; k.ny = h->ny; k.nz = h->nz; k.nf = 1;
