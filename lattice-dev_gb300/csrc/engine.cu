@@ -1659,7 +1659,8 @@ int lat_laplacian(lat_t* h, int32_t field, double* out) {
   if (!h || !out) return set_error(LAT_ERR_ARG, "null argument");
   if (field < 0 || field >= h->nf) return set_error(LAT_ERR_ARG, "bad field index");
   ApiGuard g(h);
-  RET(ensure_stage(h, (size_t)h->nf * h->N));
+  // FP32 stencil lattices: the field and its Laplacian in FP64, side by side
+  RET(ensure_stage(h, (size_t)(!spectral(h) && h->prec != LAT_FP64 ? std::max(2, h->nf) : h->nf) * h->N));
   const void* src = (const char*)h->fld[h->cur] + (size_t)field * h->N * h->rsz;
   if (spectral(h)) {
     RET(fft_source(h, &src));
@@ -1680,11 +1681,7 @@ int lat_laplacian(lat_t* h, int32_t field, double* out) {
     RET(launch_to_fp64(src, nullptr, h->N, h->prec, h->stage, h->stream));
     const double e = 1.0 / (h->dx * h->dx) / h->c[4];
     double lc[4] = {h->c[0] * e, h->c[1] * e, h->c[2] * e, h->c[3] * e};
-    double* tmp = (double*)h->lap;  // FP64 needs N doubles: lap holds nf*N reals >= N doubles only in FP64
-    if (h->prec != LAT_FP64) {
-      RET(ensure_stage(h, (size_t)std::max(2, h->nf) * h->N));
-      tmp = h->stage + h->N;
-    }
+    double* tmp = h->prec == LAT_FP64 ? (double*)h->lap : h->stage + h->N;  // lap holds nf N reals of the field's type
     RET(launch_fd_laplacian64(h->stage, tmp, h->nx, h->ny, h->nz, lc, h->stream));
     CK(cudaMemcpyAsync(out, tmp, sizeof(double) * h->N, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
