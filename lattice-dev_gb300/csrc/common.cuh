@@ -345,6 +345,16 @@ __device__ __forceinline__ void kahan_add(float& x, float& c, float inc) {
   x = t;
 }
 
+__device__ __forceinline__ double widen(double v) { return v; }
+// FP32 to FP64 by integer operations (a hardware conversion runs at the FP64 rate)
+__device__ __forceinline__ double widen(float v) {
+  const unsigned int b = __float_as_uint(v), e = (b >> 23) & 0xff;
+  if (e == 0 || e == 255) return (double)v;
+  const unsigned long long r = ((unsigned long long)(b & 0x80000000u) << 32) |
+                               ((unsigned long long)(e + 896) << 52) | ((unsigned long long)(b & 0x7fffffu) << 29);
+  return __longlong_as_double((long long)r);
+}
+
 // folded frequency |k| index of a DFT index i0 in [0,n)
 __device__ __forceinline__ int fold_idx(int i0, int n) { return i0 <= n / 2 ? i0 : n - i0; }
 

@@ -1051,7 +1051,6 @@ int compute_energies(lat_s* h, double* out, double ball_r2 = 0.0, double* ball =
   e.dx = h->dx;
   e.nx = h->nx; e.ny = h->ny; e.nz = h->nz; e.nf = h->nf;
   e.phi = h->fld[h->cur];
-  e.phic = h->fldc;
   e.pi = h->fldp;
   e.u = h->cfg.gw ? h->u[h->ucur] : nullptr;
   e.pu = h->cfg.gw ? h->pu : nullptr;
@@ -1063,7 +1062,6 @@ int compute_energies(lat_s* h, double* out, double ball_r2 = 0.0, double* ball =
   // the sums' own grid: the tuned one is the pointwise passes', and a launch of
   // one block an SM takes a third longer (256^3 FP64: 425 us against 321)
   e.grid = 4 * h->nsm;
-  e.block = 256;
   {
     Timed t(h, LAT_K_OTHER);
     RET(launch_energy(e, h->prec, h->stream));
@@ -1422,12 +1420,12 @@ int lat_create(lat_t** out, const lat_config* cfg) {
   if (spectral(h)) {
     auto cols = [&](int n) {  // x-columns per block of a y or z pass of length n
       switch (n) {
-        case 16: return sep_columns_16(h->prec, h->nf);
-        case 32: return sep_columns_32(h->prec, h->nf);
-        case 64: return sep_columns_64(h->prec, h->nf);
-        case 128: return sep_columns_128(h->prec, h->nf);
-        case 256: return sep_columns_256(h->prec, h->nf);
-        default: return sep_columns_512(h->prec, h->nf);
+        case 16: return sep_columns_16(h->nf);
+        case 32: return sep_columns_32(h->nf);
+        case 64: return sep_columns_64(h->nf);
+        case 128: return sep_columns_128(h->nf);
+        case 256: return sep_columns_256(h->nf);
+        default: return sep_columns_512(h->nf);
       }
     };
     h->sep_ok = fx_side(h->nx) && fx_side(h->ny) && fx_side(h->nz);

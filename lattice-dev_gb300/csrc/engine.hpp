@@ -242,12 +242,12 @@ struct SepFinArgs {
   KickW next;          // the next kick of the call, whose coefficients the finalize leaves in sc->co
 };
 int launch_sep_finalize(const SepFinArgs& f, cudaStream_t s);
-int sep_columns_16(int precision, int nf);
-int sep_columns_32(int precision, int nf);
-int sep_columns_64(int precision, int nf);
-int sep_columns_128(int precision, int nf);
-int sep_columns_256(int precision, int nf);
-int sep_columns_512(int precision, int nf);
+int sep_columns_16(int nf);
+int sep_columns_32(int nf);
+int sep_columns_64(int nf);
+int sep_columns_128(int nf);
+int sep_columns_256(int nf);
+int sep_columns_512(int nf);
 
 // k-space multiply F *= -k^2/N with the Parseval sum of k^2|F|^2 (Hermitian
 // weights) into sc->ge2 when store_ge2 is set.
@@ -284,7 +284,6 @@ int launch_from_fp64(const double* in, int64_t n, int precision, void* hi, void*
 struct EnergyArgs {
   int nx, ny, nz, nf;
   const void* phi;
-  const void* phic;
   const void* pi;
   const void* u;
   const void* pu;
@@ -297,7 +296,7 @@ struct EnergyArgs {
   ModelP model;
   DevScalars* sc;
   RedBuf rb;
-  int grid, block;
+  int grid;            // blocks of 256 threads: four an SM (a launch takes no more than its sums need)
   int64_t t_lo, t_hi;  // sites [t_lo, t_hi) are summed (t_hi = 0: all); a z-slab sums its interior planes
 };
 int launch_energy(const EnergyArgs& a, int precision, cudaStream_t s);

@@ -104,32 +104,32 @@ LAT_HD void cmul(i64& xr, i64& xi, const Tw& w) {
   xi = shl(hi, 2) + (mi >> 30);
 }
 
-// (xr, xi) *= exp(-+ 2 pi i J / 192) (INV: +)
+// (xr, xi) *= exp(-+ 2 pi i J / 32) (INV: +)
 template <int J0, bool INV>
 LAT_HD void cmul_const(i64& xr, i64& xi) {
-  constexpr int J = ((INV ? 192 - J0 % 192 : J0) % 192 + 192) % 192;
+  constexpr int J = ((INV ? 32 - J0 % 32 : J0) % 32 + 32) % 32;
   if constexpr (J == 0) {
     return;
-  } else if constexpr (J == 48) {  // -i
+  } else if constexpr (J == 8) {  // -i
     const i64 t = xr;
     xr = xi;
     xi = -t;
-  } else if constexpr (J == 96) {
+  } else if constexpr (J == 16) {
     xr = -xr;
     xi = -xi;
-  } else if constexpr (J == 144) {  // i
+  } else if constexpr (J == 24) {  // i
     const i64 t = xr;
     xr = -xi;
     xi = t;
-  } else if constexpr (J % 48 == 24) {
-    constexpr int ch = split_hi(kCos192[24]), cl = split_lo(kCos192[24]);
+  } else if constexpr (J % 8 == 4) {
+    constexpr int ch = split_hi(kCos32[4]), cl = split_lo(kCos32[4]);
     const i64 s = rmul(xr + xi, ch, cl), d = rmul(xi - xr, ch, cl);  // exp(-i pi/4): (s, d)
-    if constexpr (J == 24) { xr = s; xi = d; }
-    else if constexpr (J == 72) { xr = d; xi = -s; }   // times -i
-    else if constexpr (J == 120) { xr = -s; xi = -d; }
+    if constexpr (J == 4) { xr = s; xi = d; }
+    else if constexpr (J == 12) { xr = d; xi = -s; }   // times -i
+    else if constexpr (J == 20) { xr = -s; xi = -d; }
     else { xr = -d; xi = s; }
   } else {
-    constexpr i64 c = kCos192[J], s = kCos192[(J + 48) % 192];  // -sin(2 pi J/192) = cos(2 pi (J + 48)/192)
+    constexpr i64 c = kCos32[J], s = kCos32[(J + 8) % 32];  // -sin(2 pi J/32) = cos(2 pi (J + 8)/32)
     constexpr Tw w{split_hi(c), split_lo(c), split_hi(s), split_lo(s)};
     cmul<false>(xr, xi, w);
   }
@@ -166,62 +166,36 @@ LAT_HD void dft4(i64& ar, i64& ai, i64& br, i64& bi, i64& cr, i64& ci, i64& dr, 
   }
 }
 
-// 3-point DFT: X0 = a + s, X1,2 = a - s/2 -+ i (sqrt(3)/2)(b - c), s = b + c
-template <bool INV>
-LAT_HD void dft3(i64& ar, i64& ai, i64& br, i64& bi, i64& cr, i64& ci) {
-  constexpr int h = split_hi(kCos192[16]), l = split_lo(kCos192[16]);  // cos(pi/6) = sqrt(3)/2
-  const i64 sr = br + cr, si = bi + ci;
-  const i64 dr = rmul(br - cr, h, l), di = rmul(bi - ci, h, l);
-  const i64 tr = ar - (sr >> 1), ti = ai - (si >> 1);
-  ar += sr;
-  ai += si;
-  if (INV) {
-    br = tr - di;
-    bi = ti + dr;
-    cr = tr + di;
-    ci = ti - dr;
-  } else {
-    br = tr + di;
-    bi = ti - dr;
-    cr = tr - di;
-    ci = ti + dr;
-  }
-}
-
-// In-register DFT of R points, natural order in and out: radix 4 (or 3, 2)
-// by decimation in time, R = 2^k <= 64 or 3 x 2^k <= 96.
+// In-register DFT of R = 2 ... 32 points (a power of two), natural order in and
+// out: radix 4 (or 2) by decimation in time.
 template <int R, bool INV>
 LAT_HD void dft(i64 (&re)[R], i64 (&im)[R]) {
-  static_assert(192 % R == 0, "twiddles come from the 192-point table");
-  if constexpr (R == 1) {
-  } else if constexpr (R == 2) {
+  static_assert(32 % R == 0, "twiddles come from the 32-point table");
+  if constexpr (R == 2) {
     const i64 a = re[0], b = im[0];
     re[0] = a + re[1];
     im[0] = b + im[1];
     re[1] = a - re[1];
     im[1] = b - im[1];
-  } else if constexpr (R == 3) {
-    dft3<INV>(re[0], im[0], re[1], im[1], re[2], im[2]);
   } else if constexpr (R == 4) {
     dft4<INV>(re[0], im[0], re[1], im[1], re[2], im[2], re[3], im[3]);
   } else {
-    constexpr int B = R % 3 == 0 ? 3 : 4, M = R / B;  // B interleaved subsequences of M points
-    i64 sr[B][M], si[B][M];
-    static_for<B>([&](auto b) {
+    constexpr int M = R / 4;  // four interleaved subsequences of M points
+    i64 sr[4][M], si[4][M];
+    static_for<4>([&](auto b) {
       static_for<M>([&](auto k) {
-        sr[b.value][k.value] = re[B * k.value + b.value];
-        si[b.value][k.value] = im[B * k.value + b.value];
+        sr[b.value][k.value] = re[4 * k.value + b.value];
+        si[b.value][k.value] = im[4 * k.value + b.value];
       });
       dft<M, INV>(sr[b.value], si[b.value]);
       static_for<M>([&](auto k) {
-        cmul_const<(192 / R) * b.value * k.value, INV>(sr[b.value][k.value], si[b.value][k.value]);
+        cmul_const<(32 / R) * b.value * k.value, INV>(sr[b.value][k.value], si[b.value][k.value]);
       });
     });
     static_for<M>([&](auto kk) {
       constexpr int k = kk.value;
-      if constexpr (B == 3) dft3<INV>(sr[0][k], si[0][k], sr[1][k], si[1][k], sr[2][k], si[2][k]);
-      else dft4<INV>(sr[0][k], si[0][k], sr[1][k], si[1][k], sr[2][k], si[2][k], sr[B - 1][k], si[B - 1][k]);
-      static_for<B>([&](auto b) {
+      dft4<INV>(sr[0][k], si[0][k], sr[1][k], si[1][k], sr[2][k], si[2][k], sr[3][k], si[3][k]);
+      static_for<4>([&](auto b) {
         re[k + M * b.value] = sr[b.value][k];
         im[k + M * b.value] = si[b.value][k];
       });

@@ -30,16 +30,6 @@ namespace {
 enum { BIN_POWER = 0, BIN_COUNT = 1, BIN_CROSS = 2, BIN_GW = 3 };
 template <int KIND> struct Sums { static constexpr int NS = KIND == BIN_POWER ? 2 : (KIND == BIN_CROSS ? 4 : 1); };
 
-__device__ __forceinline__ double widen(double v) { return v; }
-// FP32 to FP64 by integer operations (a hardware conversion runs at the FP64 rate)
-__device__ __forceinline__ double widen(float v) {
-  const unsigned int b = __float_as_uint(v), e = (b >> 23) & 0xff;
-  if (e == 0 || e == 255) return (double)v;
-  const unsigned long long r = ((unsigned long long)(b & 0x80000000u) << 32) |
-                               ((unsigned long long)(e + 896) << 52) | ((unsigned long long)(b & 0x7fffffu) << 29);
-  return __longlong_as_double((long long)r);
-}
-
 // sum_ij |h^TT_ij|^2 of one mode: with e1, e2 normal to k,
 // 1/2 |e1 h e1 - e2 h e2|^2 + 2 |e1 h e2|^2, written out for
 // e1 = (-ky, kx, 0)/rho, e2 = (-kx kz, -ky kz, rho^2)/(rho k), rho^2 = kx^2 + ky^2

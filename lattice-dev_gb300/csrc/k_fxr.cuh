@@ -22,14 +22,6 @@ struct RowIn {
   const float* c;
 };
 
-// FP32 to FP64 by integer operations (a hardware conversion runs at the FP64 rate)
-__device__ __forceinline__ double widen(float v) {
-  const unsigned int b = __float_as_uint(v), e = (b >> 23) & 0xff;
-  if (e == 0 || e == 255) return (double)v;
-  const u64 r = ((u64)(b & 0x80000000u) << 32) | ((u64)(e + 896) << 52) | ((u64)(b & 0x7fffffu) << 29);
-  return bits_double(r);
-}
-
 template <bool F32>
 __device__ __forceinline__ double row_value(const RowIn& in, int64_t i) {
   if constexpr (F32) {

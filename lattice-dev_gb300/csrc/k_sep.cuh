@@ -685,8 +685,7 @@ int sep_dispatch(const SepArgs& a, int axis, cudaStream_t s) {
 
 // real x-columns one block of a y or z pass covers (nx must be a multiple)
 template <int N>
-int sep_columns(int precision, int nf) {
-  if (precision == LAT_FP64) return nf == 2 ? Tile<double, 2, 2, N>::W : Tile<double, 1, 2, N>::W;
+int sep_columns(int nf) {
   return nf == 2 ? Tile<float, 2, 2, N>::W : Tile<float, 1, 2, N>::W;
 }
 

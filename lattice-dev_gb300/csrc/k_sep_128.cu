@@ -9,7 +9,7 @@ int launch_sep_128(const SepArgs& a, int axis, cudaStream_t s) {
   return sep::sep_dispatch<128>(a, axis, s);
 }
 int sep_stream_lines_128(int axis) { return sep::stream_lines<128>(axis); }
-int sep_columns_128(int precision, int nf) { return sep::sep_columns<128>(precision, nf); }
+int sep_columns_128(int nf) { return sep::sep_columns<128>(nf); }
 // pairs of one-field runs (ensembles)
 int launch_sep_runs_128(const SepArgs& a, int axis, cudaStream_t s) {
   return sep::sep_stream_dispatch<128, true>(a, axis, s);

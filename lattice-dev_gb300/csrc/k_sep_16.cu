@@ -5,5 +5,5 @@ namespace lat {
 int launch_sep_16(const SepArgs& a, int axis, cudaStream_t s) {
   return sep::sep_dispatch<16>(a, axis, s);
 }
-int sep_columns_16(int precision, int nf) { return sep::sep_columns<16>(precision, nf); }
+int sep_columns_16(int nf) { return sep::sep_columns<16>(nf); }
 }  // namespace lat

@@ -9,7 +9,7 @@ int launch_sep_256(const SepArgs& a, int axis, cudaStream_t s) {
   return sep::sep_dispatch<256>(a, axis, s);
 }
 int sep_stream_lines_256(int axis) { return sep::stream_lines<256>(axis); }
-int sep_columns_256(int precision, int nf) { return sep::sep_columns<256>(precision, nf); }
+int sep_columns_256(int nf) { return sep::sep_columns<256>(nf); }
 // pairs of one-field runs (ensembles)
 int launch_sep_runs_256(const SepArgs& a, int axis, cudaStream_t s) {
   return sep::sep_stream_dispatch<256, true>(a, axis, s);

@@ -5,7 +5,7 @@ namespace lat {
 int launch_sep_64(const SepArgs& a, int axis, cudaStream_t s) {
   return sep::sep_dispatch<64>(a, axis, s);
 }
-int sep_columns_64(int precision, int nf) { return sep::sep_columns<64>(precision, nf); }
+int sep_columns_64(int nf) { return sep::sep_columns<64>(nf); }
 // pairs of one-field runs (ensembles)
 int launch_sep_runs_64(const SepArgs& a, int axis, cudaStream_t s) {
   return sep::sep_stream_dispatch<64, true>(a, axis, s);
