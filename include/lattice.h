@@ -100,11 +100,13 @@ typedef struct lat_config {
 
 /* How a spectral kick computes its Laplacian.  CUFFT: 3D R2C, -k^2/N multiply
  * and C2R (any size).  SEPARABLE: three passes of in-register 1D transforms,
- * one per axis (sides 16..512, powers of two), which also transform the FP32
- * field with its Kahan compensation.  AUTO: until lat_autotune times both on
- * the handle's lattice and keeps the faster, FP64 lattices whose sides are 9..256
- * or powers of two up to 512 run the passes (one field: more than 32^3 sites),
- * all others cuFFT. */
+ * one per axis, which also transform the FP32 field with its Kahan
+ * compensation; sides are powers of two, 16..512, and nx holds whole blocks of
+ * columns (two fields: 64 where ny or nz is 16 or 32, else 32 where one is 64 or
+ * 128, else 16; one field: twice that), other lattices are refused.  AUTO: FP64
+ * lattices whose sides are 9..256 or powers of two up to 512 run the passes (one
+ * field: more than 32^3 sites), all others cuFFT, until lat_autotune times both
+ * and keeps the faster (where SEPARABLE is accepted, or AUTO runs the passes). */
 enum lat_spectral_impl { LAT_SPEC_IMPL_AUTO = 0, LAT_SPEC_IMPL_CUFFT = 1, LAT_SPEC_IMPL_SEPARABLE = 2 };
 
 typedef struct lat_s lat_t;

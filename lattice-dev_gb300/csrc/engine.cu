@@ -247,10 +247,13 @@ bool fx_side(int n) { return n >= 16 && n <= 512 && (n & (n - 1)) == 0; }
 // two expanding fields: 0.11 ms against 0.24 ms on cuFFT at 32^3, 4.7 against
 // 24.8 at 256^3) or padded (a kick of two expanding fields: 33 us against 64 at
 // 24^3, 370 against 929 at 150 x 108 x 96, 2.2 ms against 3.8 at 192^3, the
-// least favourable side, 472 us against 4096 at 127 x 131 x 113).  One-field
-// lattices of up to 32^3 sites keep cuFFT, which AUTO has always reported for
-// them; so do FP32 lattices, whose passes round their fields differently
-// (lat_autotune or SEPARABLE choose them).
+// least favourable side, 472 us against 4096 at 127 x 131 x 113).
+// One field of up to 32^3 sites is left out, and by the autotuner too: AUTO is
+// specified to run cuFFT there (lat_spectral_impl), which is not the faster of
+// the two (a kick: 23 us on the passes against 54 on cuFFT at 32^3, 25 against
+// 48 at 30^3, 17 against 33 at 16^3, 19 against 25 at 12^3).
+// FP32 lattices stay on cuFFT until lat_autotune or SEPARABLE choose their
+// passes, which round the fields differently.
 bool auto_separable(const lat_s* h) {
   return h->fx_ok && (h->nf == 2 || h->N > 32768) && !getenv_flag("LAT_NO_SEPARABLE");
 }
@@ -1432,7 +1435,7 @@ int lat_create(lat_t** out, const lat_config* cfg) {
     // the passes need whole column blocks and (one field) an even number of x-rows
     if (h->sep_ok) h->sep_ok = h->nx % cols(h->ny) == 0 && h->nx % cols(h->nz) == 0;
     if (cfg->spectral_impl == LAT_SPEC_IMPL_SEPARABLE && !h->sep_ok)
-      return bail(set_error(LAT_ERR_UNSUPPORTED, "separable spectral passes need power-of-two sides 16..512"));
+      return bail(set_error(LAT_ERR_UNSUPPORTED, "separable spectral passes need power-of-two sides 16..512 and whole blocks of x-columns"));
     h->sep = h->sep_ok && cfg->spectral_impl == LAT_SPEC_IMPL_SEPARABLE && !getenv_flag("LAT_NO_SEPARABLE");
     // two FP32 fields on lines of 128 or 256 points whose passes all form
     // whole tiles: the streamed passes (LAT_SEP_CLASSIC=1 keeps the others)
