@@ -20,10 +20,13 @@
 // below sqrt(2) N times the line's largest value, which the multiplier's
 // `drop` bits keep below 2^62.  Nothing overflows and no stage is rescaled.
 //
-// Error.  The line enters with an absolute rounding of 2^-54 to 2^-57 of its
-// largest deviation and each product rounds to one unit of the growing
-// spectrum, whose relative weight falls with every stage; the FP64 transform
-// rounds every operation to 2^-53 of its result.
+// Error.  The line enters with an absolute rounding of one unit, less than
+// N 2^-60 of its largest deviation: 2^-54 to 2^-57 of it on noise, 2^-51 where
+// 512 deviations are of one size.  Each product rounds to one unit of the
+// growing spectrum, whose relative weight falls with every stage; the FP64
+// transform rounds every operation to 2^-53 of its result.  The derivative's
+// error stays below 8 2^-53 of the largest that such a line can have
+// (tests/test_fx_lines.py).
 //
 // A product x w with w = W 2^-62: x = xh 2^32 + xl and W = Wh 2^32 + Wl with
 // signed low halves, x W 2^-62 = (xh Wh) 4 + (xh Wl + xl Wh) 2^-30 + (xl Wl)

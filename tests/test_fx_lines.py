@@ -120,6 +120,26 @@ def test_line_against_long_double(fx, n, padded, kind):
     assert worst[0] <= 1.1 * worst[1] + 8 * 2.0 ** -53
 
 
+@pytest.mark.parametrize("kind", ["uneven", "tiny", "large"])
+@pytest.mark.parametrize("n,padded", [(n, False) for n in SIZES] + [(n, True) for n in PADDED])
+def test_either_line_of_an_uneven_pair(fx, n, padded, kind):
+    """Each line of a pair of very different size, against the FP64 transform of that line alone: its own
+    exponent keeps it as exact as a line of a like pair."""
+    rng = np.random.default_rng(100 + n)
+    c = kernel(n)
+    worst = np.zeros((2, 2))
+    for _ in range(4):
+        pair = inputs(n, kind, rng)
+        out = fx(*pair, padded=padded)
+        for l, x in enumerate(pair):
+            e = exact(x, c)
+            norm = np.sqrt(np.sum(e * e))
+            alone = fp64(x, np.zeros(n))[0]
+            worst[l] += [float(np.sqrt(np.sum((v - e) ** 2)) / norm) for v in (out[l], alone)]
+    for l in (0, 1):
+        assert worst[l][0] <= 1.1 * worst[l][1] + 8 * 2.0 ** -53, l
+
+
 @pytest.mark.parametrize("n,padded", [(n, False) for n in SIZES] + [(n, True) for n in PADDED])
 def test_line_special_values(fx, n, padded):
     fx = functools.partial(fx, padded=padded)
