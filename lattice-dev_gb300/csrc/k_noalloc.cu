@@ -69,6 +69,9 @@ __global__ void __launch_bounds__(256) na_spec_kernel(NaArgs a) {
     const unsigned int r = m / hx;
     const int y = (int)(r % ny), z = (int)(r / ny);
     const int jj = na_fold(y, a.ny), kk = na_fold(z, a.nz);
+    // beyond the last shell; what is left keeps |n|^2 below 3 nb^2, also on a box
+    // whose side's square is beyond 32 bits
+    if (x >= nb || jj >= nb || kk >= nb) continue;
     const double wx = (x == 0 || 2 * x == a.nx) ? 1.0 : 2.0;
     const int m2 = x * x + jj * jj + kk * kk;
     const int l = na_isqrt(m2);

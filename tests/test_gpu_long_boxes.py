@@ -53,6 +53,29 @@ def test_spectra(engine, shape, nb):
     g.close()
 
 
+@pytest.mark.parametrize("mode", [L.SPEC_WEIGHTED, L.SPEC_COUNT])
+@pytest.mark.parametrize("shape", [(8200, 4, 2), (131072, 2, 2), (2, 131072, 2), (2, 2, 131072)])
+def test_noalloc_spectra(engine, shape, mode):
+    """The allocation-free binning of the same transform: sums in another order."""
+    torch = pytest.importorskip("torch")
+    nx, ny, nz = shape
+    nb = 300
+    g = engine.Lattice(L.make_config(shape, nfld=1, length=1.0, laplacian=L.LAP_FD7, precision=L.FP64,
+                                     model=L.MODEL_PHI4, model_params=(1.0,)))
+    f, p = random_state((1, nz, ny, nx), seed=3, mean=0.2, amp=1.0)
+    g.set_state(f, p)
+    S, W = g.spectrum(L.SPEC_FLD, 0, mode, nb)
+    F = torch.from_numpy(np.fft.rfftn(f[0])).cuda().contiguous()
+    out = torch.zeros(2 * nb, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert engine._lib.lat_spectrum_noalloc(F.data_ptr(), nx, ny, nz, L.FP64, mode, nb, out.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    assert np.allclose(got[nb:], W, rtol=1e-12, atol=0)
+    assert np.all(np.abs(got[:nb] - S) <= 1e-11 * (S + np.mean(S)))
+    g.close()
+
+
 def neighbours(g, lap):
     """Sums over the 6 face and, with 27 points, 12 edge and 8 corner neighbours."""
     n = lambda v, d: np.roll(v, 1, d) + np.roll(v, -1, d)  # noqa: E731
