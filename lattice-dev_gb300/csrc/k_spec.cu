@@ -327,7 +327,9 @@ __global__ void __launch_bounds__(256) kmul_kernel(KmulArgs a) {
     const unsigned int r = mm / hxu;
     const int y = (int)(r % nyu), z = (int)(r / nyu);
     const int jj = fold_idx(y, a.ny), kk = fold_idx(z, a.nz);
-    const R k2 = (R)(x * x) * dkx2 + (R)(jj * jj) * dky2 + (R)(kk * kk) * dkz2;
+    // whole numbers whose squares may be beyond 32 bits (sides from 92682 points on)
+    const R xr = (R)x, yr = (R)jj, zr = (R)kk;
+    const R k2 = xr * xr * dkx2 + yr * yr * dky2 + zr * zr * dkz2;
     C v = F[m];
     if (a.store_ge2) {
       const R w = (x == 0 || 2 * x == a.nx) ? R(1) : R(2);

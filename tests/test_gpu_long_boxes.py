@@ -76,6 +76,34 @@ def test_noalloc_spectra(engine, shape, mode):
     g.close()
 
 
+@pytest.mark.parametrize("prec,tol", [(L.FP64, 1e-12), (L.FP32_KAHAN, 1e-5)])
+@pytest.mark.parametrize("shape", [(131072, 2, 2), (2, 131072, 2), (2, 2, 131072)])
+def test_spectral_laplacian(engine, shape, prec, tol):
+    """Squares of mode numbers beyond 32 bits: read-out, gradient energy and one kick of a long spectral box.
+    The largest mode number is 65536; a transform's rounding is relative to the largest derivative."""
+    nx, ny, nz = shape
+    g = engine.Lattice(L.make_config(shape, nfld=1, length=1.0 * nx, laplacian=L.LAP_SPECTRAL, precision=prec,
+                                     model=L.MODEL_FREE, model_params=(0.0,)))
+    g.set_state(*random_state((1, nz, ny, nx), seed=5, mean=0.0, amp=1.0))
+    f, p = (v[0] for v in g.get_state())
+    k = [np.fft.fftfreq(n, 1.0 / n) * 2 * np.pi / n for n in (nz, ny, nx)]  # dx = 1
+    k2 = k[0][:, None, None] ** 2 + k[1][None, :, None] ** 2 + k[2][None, None, :] ** 2
+    F = np.fft.fftn(f)
+    ref = np.fft.ifftn(-k2 * F).real
+    top = np.max(np.abs(ref))
+    assert np.max(np.abs(g.laplacian() - ref)) <= tol * top
+    want = 0.5 * np.sum(k2 * np.abs(F) ** 2) / float(f.size) ** 2
+    assert abs(g.energies()[L.E_GE_LAP] - want) <= tol * want
+    dt = 0.01
+    g.symp(2, dt, 1)
+    f = f + 0.5 * dt * p
+    p = p + dt * np.fft.ifftn(-k2 * np.fft.fftn(f)).real
+    f = f + 0.5 * dt * p
+    got = g.get_state()
+    assert np.max(np.abs(got[1][0] - p)) <= tol * top and np.max(np.abs(got[0][0] - f)) <= tol * top
+    g.close()
+
+
 def neighbours(g, lap):
     """Sums over the 6 face and, with 27 points, 12 edge and 8 corner neighbours."""
     n = lambda v, d: np.roll(v, 1, d) + np.roll(v, -1, d)  # noqa: E731
