@@ -118,7 +118,7 @@ def neighbours(g, lap):
 @pytest.mark.parametrize("prec,tol", [(L.FP64, 1e-12), (L.FP32_KAHAN, 2e-5)])
 @pytest.mark.parametrize("shape,lap", [((2, 262200, 2), L.LAP_FD7), ((2, 262200, 2), L.LAP_FD27),
                                        ((3, 2, 140000), L.LAP_FD7), ((3, 2, 140000), L.LAP_FD27),
-                                       ((64, 262148, 2), L.LAP_FD27)])
+                                       ((64, 262148, 2), L.LAP_FD27), ((2, 524300, 2), L.LAP_FD27)])
 def test_stencil_step_and_energies(engine, shape, lap, prec, tol):
     """Two leapfrog steps and the energies on the untuned tile.  FP64: sums of 27 terms of order one, a few
     steps; FP32: the same to the format, energies as sums of FP32 terms."""
